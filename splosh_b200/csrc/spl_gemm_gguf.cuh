@@ -78,12 +78,18 @@ __global__ void spl_repack_gguf_kernel(const unsigned char *__restrict__ native,
     }
 }
 
-// Stages of weight blocks in flight: three, or two where the widened blocks beside 64 rows of activations would not fit
-// (as many as fit, five at 16 rows, were measured: no change, the kernel does not wait for memory).
-__host__ __device__ constexpr int spl_gguf_cstages(int rn, int format) { return (rn >= 64 && format != SPL_GGUF_Q4K) ? 2 : 3; }
+// Stages of weight blocks in flight: as many as there are dequant sets (more, five at 16 rows, were measured: no change). The
+// sets take the half-stage units in turn, so a set works in two stages of every three: with three slots it comes back to the
+// same two, and has itself seen a slot's last phase when it waits for the next. With a ring of another length it would
+// meet slots whose last phase it skipped, and where that copy was still under way (the next slot's had overtaken it) the wait for
+// the coming phase would be answered by the one before: the set would read the old tenant and hand its slot back early
+// (at two stages, 64 rows of the byte-wide types: a wrong sum, or a launch failure in the blocks after it).
+#define SPL_GG_CSTAGES 3
+// Stages of activations: four, or three where the widened blocks beside 64 rows leave no room for a fourth.
+__host__ __device__ constexpr int spl_gguf_bstages(int rn, int format) { return (rn >= 64 && format != SPL_GGUF_Q4K) ? 3 : 4; }
 #define SPL_GG_THREADS 480       // warps 0-3, 8-11 and 4-7: three dequant sets; 12 copies; 13-14 tensor-core issue
 __host__ __device__ constexpr size_t spl_gguf_smem_bytes(int rn, int format) {
-    return 1024 + size_t(spl_gguf_cstages(rn, format)) * spl_gguf_pieces(format) * 2048 + size_t(4) * SPL_TC_SUPER * rn * 128 + 1024;
+    return 1024 + size_t(SPL_GG_CSTAGES) * spl_gguf_pieces(format) * 2048 + size_t(spl_gguf_bstages(rn, format)) * SPL_TC_SUPER * rn * 128 + 1024;
 }
 __device__ __forceinline__ float spl_half_bits_to_float(uint32_t bits) { return __half2float(__ushort_as_half(uint16_t(bits))); }
 // Two fp32 values -> one register of two fp16, each rounded to nearest even.
@@ -196,7 +202,7 @@ template <int RN, int FMT>
 __global__ void __launch_bounds__(SPL_GG_THREADS, 1)
 spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfloat16 *__restrict__ act, float *out, int out_ld,
                         const float *residual, float *partials, int rows, int op_blocks, int supers_total, int supers_per_split, int *error_flag) {
-    constexpr int BST = 4, CST = spl_gguf_cstages(RN, FMT), ASUP = 2, AST = 4 * ASUP, PIECES = spl_gguf_pieces(FMT);
+    constexpr int BST = spl_gguf_bstages(RN, FMT), CST = SPL_GG_CSTAGES, ASUP = 2, AST = 4 * ASUP, PIECES = spl_gguf_pieces(FMT);
     constexpr int BTILE = SPL_TC_SUPER * RN * 128, WSTAGE = PIECES * 2048;
     extern __shared__ unsigned char spl_gg_smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(spl_gg_smem_raw) + 1023) & ~uintptr_t(1023));
