@@ -130,51 +130,118 @@ spl_argmax_kernel(const float *__restrict__ logits, int ld, int limit, int32_t *
 }
 
 // The k largest of [0, limit) per logit row in descending order, the lower index first among equal values
-// (TopK.select, Sampler.swift:19-52). k rounds of a block-wide selection: round r takes the best element that comes
-// strictly after the previous pick in the order (value descending, index ascending); the row stays in L2 between rounds.
-// Grid (rows), 1024 threads; ids and values [rows][k].
-__global__ void __launch_bounds__(1024)
-spl_topk_kernel(const float *__restrict__ logits, int ld, int limit, int k, int32_t *ids, float *values) {
-    __shared__ float best_v[32];
-    __shared__ int best_i[32];
-    __shared__ float pick_v;
-    __shared__ int pick_i;
-    const float *x = logits + size_t(blockIdx.x) * ld;
-    float last_v = INFINITY; int last_i = -1;
+// (TopK.select, Sampler.swift:19-52), in two kernels, so that a row is many blocks' work and is read once. A warp keeps a
+// stretch of 1,024 values in registers as order-preserving keys (32 a lane, in four groups with a maximum each) and picks k
+// times: two warp-wide reductions find the best key and its lowest index, and the lane that held it looks for its next
+// best in one group. A block merges its eight sorted lists; the second kernel merges a row's blocks the same way, a lane a
+// list. Bound: the row's one trip from HBM for many rows, the chain of k picks for few.
+// One block a row scanning it k times (what this replaced) took 1.31-1.34 ms for k = 20 of 248,077 at 12 to 64 rows.
+//
+// A key is the float's bits made to order as unsigned numbers, minus zero taken as zero (the two are equal values, so the lower
+// index goes first); 0 stands for what is never picked: NaN, -inf and what lies past the limit.
+#define SPL_TOPK_WARP 1024               // values of a warp
+#define SPL_TOPK_STRETCH (8 * SPL_TOPK_WARP)
+#define SPL_TOPK_MAX 64
+__device__ __forceinline__ uint32_t spl_topk_key(float v) {
+    if (!(v > -INFINITY)) return 0u;
+    const uint32_t b = __float_as_uint(v + 0.0f);
+    return b ^ (uint32_t(int32_t(b) >> 31) | 0x80000000u);
+}
+// k rounds of a merge of sorted lists by one warp: list n is lists[n * k ...] (key, index), ended by key 0 or by its k-th
+// entry; a lane walks the lists lane, lane + 32, ... Round r's pick (key 0: none left) goes to emit(r, key, index) on lane 0.
+template <typename Emit>
+__device__ __forceinline__ void spl_topk_merge_lists(const uint2 *lists, int count, int k, uint8_t *cursor, Emit emit) {
+    const int lane = threadIdx.x & 31;
+    uint2 head = make_uint2(0u, 0xffffffffu); int mine = -1;
+    auto next = [&]() {                                       // the best head of this lane's lists
+        head = make_uint2(0u, 0xffffffffu); mine = -1;
+        for (int n = lane; n < count; n += 32) {
+            const int at = cursor[n];
+            if (at >= k) continue;
+            const uint2 c = lists[size_t(n) * k + at];
+            if (c.x > head.x || (c.x == head.x && c.y < head.y)) { head = c; mine = n; }
+        }
+    };
+    next();
     for (int round = 0; round < k; ++round) {
-        float bv = -INFINITY; int bi = 0x7fffffff;
-        for (int i = threadIdx.x; i < limit; i += blockDim.x) {
-            const float v = x[i];
-            const bool after = v < last_v || (v == last_v && i > last_i);          // not taken in an earlier round (NaNs never qualify)
-            if (after && v > -INFINITY && (v > bv || (v == bv && i < bi))) { bv = v; bi = i; }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-        }
-        if ((threadIdx.x & 31) == 0) { best_v[threadIdx.x >> 5] = bv; best_i[threadIdx.x >> 5] = bi; }
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            bv = best_v[threadIdx.x]; bi = best_i[threadIdx.x];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-            }
-            if (threadIdx.x == 0) {
-                // Fewer than k selectable values (a short row, NaNs, -inf): the reference's untouched slots, id 0 at -inf.
-                const bool none = bi == 0x7fffffff;
-                pick_v = none ? -INFINITY : bv; pick_i = none ? -1 : bi;
-                ids[size_t(blockIdx.x) * k + round] = none ? 0 : bi; values[size_t(blockIdx.x) * k + round] = pick_v;
-            }
-        }
-        __syncthreads();
-        if (pick_i < 0) { last_v = -INFINITY; last_i = 0x7ffffffe; } else { last_v = pick_v; last_i = pick_i; }
-        __syncthreads();
+        const uint32_t key = __reduce_max_sync(0xffffffffu, head.x);
+        const uint32_t index = __reduce_min_sync(0xffffffffu, head.x == key ? head.y : 0xffffffffu);
+        if (lane == 0) emit(round, key, index);
+        if (key != 0u && head.x == key && head.y == index) { ++cursor[mine]; next(); }
     }
+}
+// Grid (stretches, rows), 256 threads; lists [rows][stretches][k] of (key, index).
+__global__ void __launch_bounds__(256)
+spl_topk_stretch_kernel(const float *__restrict__ logits, int ld, int limit, int k, uint2 *lists) {
+    __shared__ uint2 own[8 * SPL_TOPK_MAX];
+    __shared__ uint8_t cursor[8];
+    spl_grid_begin();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int base = int(blockIdx.x) * SPL_TOPK_STRETCH + warp * SPL_TOPK_WARP + lane;
+    const float *x = logits + size_t(blockIdx.y) * ld;
+    float v[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) v[e] = base + 32 * e < limit ? x[base + 32 * e] : -INFINITY;
+    uint32_t key[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) key[e] = spl_topk_key(v[e]);
+    uint32_t taken = 0u;                                      // this lane's elements that have been picked
+    auto group = [&](int q) {
+        uint32_t m = 0u;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) m = max(m, (taken >> (8 * q + e) & 1u) ? 0u : key[8 * q + e]);
+        return m;
+    };
+    // (the groups are spelt out: a loop over them becomes an indexed array in local memory)
+    uint32_t top0 = group(0), top1 = group(1), top2 = group(2), top3 = group(3);
+    uint2 *list = own + warp * k;
+    for (int round = 0; round < k; ++round) {
+        const uint32_t best = max(max(top0, top1), max(top2, top3));
+        const uint32_t all = __reduce_max_sync(0xffffffffu, best);
+        if (all == 0u) {                                      // nothing left: the list ends here
+            if (lane == 0) list[round] = make_uint2(0u, 0xffffffffu);
+            break;
+        }
+        // The lowest element of this lane that has the key (elements ascend in index), and the lowest index of the warp.
+        int e0 = 32;
+        if (best == all) {
+#pragma unroll
+            for (int e = 31; e >= 0; --e) e0 = (key[e] == all && !(taken >> e & 1u)) ? e : e0;
+        }
+        const uint32_t at = uint32_t(base + 32 * e0);
+        const uint32_t first = __reduce_min_sync(0xffffffffu, e0 < 32 ? at : 0xffffffffu);
+        if (e0 < 32 && at == first) {
+            list[round] = make_uint2(all, first);
+            taken |= 1u << e0;
+            if (e0 < 16) { if (e0 < 8) top0 = group(0); else top1 = group(1); }
+            else { if (e0 < 24) top2 = group(2); else top3 = group(3); }
+        }
+    }
+    if (lane == 0) cursor[warp] = 0;
+    __syncthreads();
+    if (warp != 0) return;
+    // A list that ended early has key 0 at its end and is not read beyond it: a pick never has key 0.
+    uint2 *out = lists + (size_t(blockIdx.y) * gridDim.x + blockIdx.x) * k;
+    spl_topk_merge_lists(own, 8, k, cursor, [&](int round, uint32_t picked, uint32_t index) { out[round] = make_uint2(picked, index); });
+}
+// Grid (rows), 32 threads; ids and values [rows][k]. Dynamic shared memory: a cursor byte a list, after the row's lists where
+// `staged` (they fit the default 48 KB up to 95 stretches at k = 64: the k picks then wait for shared memory instead of L2).
+// Fewer than k selectable values (a short row, NaNs, -inf) leave the reference's untouched slots, id 0 at -inf.
+__global__ void __launch_bounds__(32)
+spl_topk_merge_kernel(const float *__restrict__ logits, int ld, const uint2 *lists, int count, int k, int staged, int32_t *ids, float *values) {
+    extern __shared__ uint2 spl_topk_smem[];
+    spl_grid_begin();
+    const int lane = threadIdx.x;
+    const uint2 *row_lists = lists + size_t(blockIdx.x) * count * k;
+    uint8_t *cursor = reinterpret_cast<uint8_t *>(spl_topk_smem + (staged ? count * k : 0));
+    if (staged) for (int i = lane; i < count * k; i += 32) spl_topk_smem[i] = row_lists[i];
+    for (int n = lane; n < count; n += 32) cursor[n] = 0;
+    __syncwarp();
+    spl_topk_merge_lists(staged ? spl_topk_smem : row_lists, count, k, cursor, [&](int round, uint32_t picked, uint32_t index) {
+        const size_t at = size_t(blockIdx.x) * k + round;
+        ids[at] = picked ? int32_t(index) : 0;
+        values[at] = picked ? logits[size_t(blockIdx.x) * ld + index] : -INFINITY;
+    });
 }
 
 // Fill helpers for synthetic contexts.

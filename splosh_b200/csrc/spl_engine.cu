@@ -80,7 +80,7 @@ struct spl_engine {
     // Drafter feature taps (Engine.swift:330-331, 1488-1497): the residual stream after the listed blocks, [row][tap][hidden].
     float *features = nullptr;
     std::vector<int> feature_layers;
-    int32_t *topk_ids = nullptr; float *topk_values = nullptr;      // allocated by the first spl_topk
+    uint2 *topk_lists = nullptr; int32_t *topk_picks = nullptr, *topk_host = nullptr;      // allocated by the first spl_topk
     __half *q = nullptr;
     int32_t *argmax_ids = nullptr;
     int proj_ld = 0, gate_up_ld = 0, core_ld = 0, logits_ld = 0;
@@ -920,7 +920,7 @@ void spl_engine_destroy(spl_engine *e) {
     for (auto p : e->state) cudaFree(p); for (auto p : e->conv) cudaFree(p); for (auto p : e->journal) cudaFree(p);
     cudaFree(e->h); cudaFree(e->xn); cudaFree(e->proj); cudaFree(e->gdn_act); cudaFree(e->core); cudaFree(e->gate_up); cudaFree(e->act);
     cudaFree(e->q); cudaFree(e->hsn); cudaFree(e->logits); cudaFree(e->argmax_ids); cudaFree(e->partials); cudaFree(e->attn_partials);
-    cudaFree(e->taps); cudaFree(e->features); cudaFree(e->topk_ids); cudaFree(e->topk_values); cudaFree(e->tables_dev); cudaFree(e->gdn_records); cudaFree(e->gdn_o_raw); cudaFree(e->slots); cudaFree(e->xn_squares); cudaFree(e->xn_sums); cudaFree(e->core_sums); cudaFree(e->act_sums); cudaFree(e->hsn_sums); cudaFree(e->tc_error);
+    cudaFree(e->taps); cudaFree(e->features); cudaFree(e->topk_lists); cudaFree(e->topk_picks); cudaFreeHost(e->topk_host); cudaFree(e->tables_dev); cudaFree(e->gdn_records); cudaFree(e->gdn_o_raw); cudaFree(e->slots); cudaFree(e->xn_squares); cudaFree(e->xn_sums); cudaFree(e->core_sums); cudaFree(e->act_sums); cudaFree(e->hsn_sums); cudaFree(e->tc_error);
     if (e->tables_host) cudaFreeHost(e->tables_host);
     for (ProfileSlot &s : e->profile_slots) { cudaEventDestroy(s.begin); cudaEventDestroy(s.end); }
     if (e->ev_begin) cudaEventDestroy(e->ev_begin);
@@ -1251,17 +1251,23 @@ spl_status spl_topk(spl_engine *e, int32_t vocab_limit, int32_t k, int32_t *ids,
     SPL_NOT_IN_FLIGHT(e);
     if (e->last_logit_rows == 0) return SPL_OK;
     SPL_CUDA(cudaSetDevice(e->device));
-    const size_t cells = size_t(e->host->config.max_logit_rows) * 64;
-    if (!e->topk_ids) {
-        SPL_CUDA(cudaMalloc(reinterpret_cast<void **>(&e->topk_ids), cells * 4));
-        SPL_CUDA(cudaMalloc(reinterpret_cast<void **>(&e->topk_values), cells * 4));
-    }
-    spl_topk_kernel<<<e->last_logit_rows, 1024, 0, e->stream>>>(e->logits, e->logits_ld, vocab_limit, k, e->topk_ids, e->topk_values);
+    // Room for every logit row at the largest k: the rows' candidate lists, and the picks (ids, then values) with a pinned copy.
+    const size_t max_rows = size_t(e->host->config.max_logit_rows), max_stretches = size_t(e->g.vocab + SPL_TOPK_STRETCH - 1) / SPL_TOPK_STRETCH;
+    if (!e->topk_lists) SPL_CUDA(cudaMalloc(reinterpret_cast<void **>(&e->topk_lists), max_rows * max_stretches * SPL_TOPK_MAX * sizeof(uint2)));
+    if (!e->topk_picks) SPL_CUDA(cudaMalloc(reinterpret_cast<void **>(&e->topk_picks), max_rows * SPL_TOPK_MAX * 8));
+    if (!e->topk_host) SPL_CUDA(cudaMallocHost(reinterpret_cast<void **>(&e->topk_host), max_rows * SPL_TOPK_MAX * 8));
+    const int rows = e->last_logit_rows, stretches = (vocab_limit + SPL_TOPK_STRETCH - 1) / SPL_TOPK_STRETCH;
+    const size_t picks = size_t(rows) * k, staged_bytes = size_t(stretches) * k * sizeof(uint2) + stretches;
+    const bool staged = staged_bytes <= 48 * 1024;
+    launch_step(spl_topk_stretch_kernel, dim3(stretches, rows), dim3(256), 0, e->stream, (const float *)e->logits, e->logits_ld, vocab_limit, k, e->topk_lists);
+    launch_step(spl_topk_merge_kernel, dim3(rows), dim3(32), staged ? staged_bytes : size_t(stretches), e->stream, (const float *)e->logits, e->logits_ld, (const uint2 *)e->topk_lists,
+                stretches, k, staged ? 1 : 0, e->topk_picks, reinterpret_cast<float *>(e->topk_picks) + picks);
     const spl_status launched = check_launch(e, "top-k");
     if (launched != SPL_OK) return launched;
-    SPL_CUDA(cudaMemcpyAsync(ids, e->topk_ids, size_t(e->last_logit_rows) * k * 4, cudaMemcpyDeviceToHost, e->stream));
-    SPL_CUDA(cudaMemcpyAsync(values, e->topk_values, size_t(e->last_logit_rows) * k * 4, cudaMemcpyDeviceToHost, e->stream));
+    SPL_CUDA(cudaMemcpyAsync(e->topk_host, e->topk_picks, picks * 8, cudaMemcpyDeviceToHost, e->stream));
     SPL_CUDA(cudaStreamSynchronize(e->stream));
+    std::memcpy(ids, e->topk_host, picks * 4);
+    std::memcpy(values, e->topk_host + picks, picks * 4);
     return SPL_OK;
 }
 

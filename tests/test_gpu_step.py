@@ -371,6 +371,45 @@ def test_topk_on_the_device_and_sampling_from_it(toks):
         engine.topk(65)
 
 
+class _SparseHead:
+    """The tiny model with a head whose rows are zero but for `kept`: every other logit is exactly zero."""
+
+    def __init__(self, model, kept):
+        self.model, self.kept = model, kept
+
+    def q4(self, layer, kind):
+        packed, scales, biases = self.model.q4(layer, kind)
+        if kind == "head":
+            scales, biases = scales.copy(), biases.copy()
+            scales[~self.kept] = 0
+            biases[~self.kept] = 0
+        return packed, scales, biases
+
+    def vec(self, layer, kind):
+        return self.model.vec(layer, kind)
+
+
+@pytest.mark.parametrize("kept", [0, 1, 30, 60, 5000])
+def test_topk_orders_equal_values_by_index_across_lanes_warps_and_stretches(toks, kept):
+    """A head of mostly zero rows: the picks run from a few distinct values into equal ones that lie in one lane, in other warps and in
+    other stretches. Limits at and around a warp's 1,024 values and a stretch's 8,192."""
+    from oracle import sampler as OS
+    g = S.tiny_geometry()
+    model = O.Model(O.tiny_geometry())
+    mask = np.zeros(g.vocab, bool)
+    mask[np.random.default_rng(kept).permutation(g.vocab)[:kept]] = True
+    engine = S.Engine(g, S.EngineConfig(max_slots=1, max_rows=32, kv_pages=2, max_context=256))
+    engine.load_model(_SparseHead(model, mask))
+    engine.step([S.EngineRow(0, toks[i], i, i >= 2) for i in range(5)])
+    logits = engine.all_logits()
+    assert (logits[:, ~mask] == 0).all()
+    for k, limit in ((64, g.vocab), (20, 8192), (20, 8193), (1, 1024), (33, 1025), (64, 64), (5, 8191), (64, 16385)):
+        ids, values = engine.topk(k, limit)
+        for r in range(logits.shape[0]):
+            rid, rvalues = OS.topk_select(logits[r], limit, k)
+            assert list(ids[r]) == rid and np.array_equal(values[r], rvalues), (k, limit, r)
+
+
 def test_a_slot_moves_to_another_engine_through_state_and_kv_snapshots(toks):
     """exportState / exportKV / importState / importSlot (Engine.swift:870-1042). A conversation of 300 tokens plus one
     accepted 6-row speculative block (so the export has journal entries to fold in) moves from slot 0 of engine A to
