@@ -243,9 +243,9 @@ bool configure_device(int device, int *sms) {
     if (device < 0 || device >= 64) return false;
     if (!done[device]) {
         configure_gemm<16>(); configure_gemm<32>(); configure_gemm<64>(); configure_gemm<128>();
-        configure_gguf<16, SPL_GGUF_Q4K>(); configure_gguf<32, SPL_GGUF_Q4K>(); configure_gguf<64, SPL_GGUF_Q4K>();
-        configure_gguf<16, SPL_GGUF_Q5K>(); configure_gguf<32, SPL_GGUF_Q5K>(); configure_gguf<64, SPL_GGUF_Q5K>();
-        configure_gguf<16, SPL_GGUF_Q6K>(); configure_gguf<32, SPL_GGUF_Q6K>(); configure_gguf<64, SPL_GGUF_Q6K>();
+        configure_gguf<16, SPL_GGUF_Q4K>(); configure_gguf<32, SPL_GGUF_Q4K>(); configure_gguf<64, SPL_GGUF_Q4K>(); configure_gguf<128, SPL_GGUF_Q4K>();
+        configure_gguf<16, SPL_GGUF_Q5K>(); configure_gguf<32, SPL_GGUF_Q5K>(); configure_gguf<64, SPL_GGUF_Q5K>(); configure_gguf<128, SPL_GGUF_Q5K>();
+        configure_gguf<16, SPL_GGUF_Q6K>(); configure_gguf<32, SPL_GGUF_Q6K>(); configure_gguf<64, SPL_GGUF_Q6K>(); configure_gguf<128, SPL_GGUF_Q6K>();
         configure_scan<256, 6>(); configure_scan<128, 4>();
         cudaFuncSetAttribute(spl_gdn_recurrence_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_gdn_recurrence_smem()));
         cudaFuncSetAttribute(spl_gdn_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_gdn_chunk_prepare_smem()));
@@ -409,7 +409,7 @@ void launch_gemm_gguf_tc(cudaStream_t stream, const SplGgufDev &w, const GemmOpe
     const int splits4 = choose_splits(w.tiles * row_blocks, supers * 4, 148, partial_floats, size_t(rows_padded) * w.ld);
     const int sps = (supers + splits4 - 1) / splits4, splits = (supers + sps - 1) / sps;
     const size_t smem = spl_gguf_smem_bytes(RN, FMT);
-    launch_step(spl_gemm_gguf_tc_kernel<RN, FMT>, dim3(w.tiles, splits, row_blocks), dim3(SPL_GG_THREADS), smem, stream,
+    launch_step(spl_gemm_gguf_tc_kernel<RN, FMT>, dim3(w.tiles * row_blocks, splits), dim3(SPL_GG_THREADS), smem, stream,
                 w.blocks, op.values, out, w.ld, residual, partials, rows, op.blocks, supers, sps, error_flag);
     if (splits > 1) {
         const size_t total = size_t(rows) * w.ld / 4;
@@ -421,7 +421,8 @@ void launch_gemm_gguf_rows(cudaStream_t stream, const SplGgufDev &w, const GemmO
                            float *partials, size_t partial_floats, int *error_flag) {
     if (op.rn == 16) launch_gemm_gguf_tc<16, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
     else if (op.rn == 32) launch_gemm_gguf_tc<32, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
-    else launch_gemm_gguf_tc<64, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
+    else if (op.rn == 64) launch_gemm_gguf_tc<64, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
+    else launch_gemm_gguf_tc<128, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
 }
 void launch_gemm_gguf(cudaStream_t stream, const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows,
                       float *partials, size_t partial_floats, int *error_flag) {
@@ -510,7 +511,7 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
 
     const int H = g.hidden;
     // GEMM operands of this step: row blocks of rn rows, in the tile layout the tensor cores read.
-    const int rn = gguf ? std::min(operand_rn(R), 64) : operand_rn(R), blocks = (R + rn - 1) / rn;      // the GGUF kernel's blocks hold up to 64 rows
+    const int rn = operand_rn(R), blocks = (R + rn - 1) / rn;
     const SplOperand xn{e->xn, e->xn_sums, rn, blocks}, core{e->core, e->core_sums, rn, blocks}, act{e->act, e->act_sums, rn, blocks};
     const GemmOperand gxn{e->xn, e->xn_sums, rn, blocks}, gcore{e->core, e->core_sums, rn, blocks}, gact{e->act, e->act_sums, rn, blocks};
     profile_begin(e, KLASS_ELEMENTWISE, 0);
@@ -637,7 +638,7 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
     }
     if (t->logit_rows > 0) {
         profile_begin(e, KLASS_OTHER, 0);
-        const int lrn = gguf ? std::min(operand_rn(int(t->logit_rows)), 64) : operand_rn(int(t->logit_rows)), lblocks = (int(t->logit_rows) + lrn - 1) / lrn;
+        const int lrn = operand_rn(int(t->logit_rows)), lblocks = (int(t->logit_rows) + lrn - 1) / lrn;
         norm(int(t->logit_rows), e->final_norm, e->d_gather, SplOperand{e->hsn, e->hsn_sums, lrn, lblocks});
         profile_end(e);
         if (gguf) ggemm(e->g_head, GemmOperand{e->hsn, e->hsn_sums, lrn, lblocks}, e->logits, nullptr, int(t->logit_rows));
@@ -1837,7 +1838,7 @@ spl_status spl_op_gemm_gguf(int32_t device, int32_t format, const uint8_t *block
     SPL_CUDA(cudaStreamCreate(&e->stream));
     SplGgufDev w;
     w.n = n; w.ld = round16(n); w.tiles = (n + 127) / 128; w.k = k; w.format = format;
-    const int ld = w.ld, rn = std::min(operand_rn(rows), 64), row_blocks = (rows + rn - 1) / rn;      // the GGUF kernel's blocks hold up to 64 rows
+    const int ld = w.ld, rn = operand_rn(rows), row_blocks = (rows + rn - 1) / rn;
     float *d_act32 = nullptr, *d_out = nullptr, *d_sums = nullptr; __nv_bfloat16 *d_act = nullptr; int *d_flag = nullptr; unsigned char *d_native = nullptr;
     e->partial_floats = size_t(16) * row_blocks * rn * ld;
     spl_status s = SPL_OK;

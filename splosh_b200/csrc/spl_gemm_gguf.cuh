@@ -85,11 +85,15 @@ __global__ void spl_repack_gguf_kernel(const unsigned char *__restrict__ native,
 // the coming phase would be answered by the one before: the set would read the old tenant and hand its slot back early
 // (at two stages, 64 rows of the byte-wide types: a wrong sum, or a launch failure in the blocks after it).
 #define SPL_GG_CSTAGES 3
-// Stages of activations: four, or three where the widened blocks beside 64 rows leave no room for a fourth.
+// The 128-row block (steps of more than 64 rows: prompt chunks) forms a weight once for twice the rows of the 64-row block. Its
+// activations come a unit (two groups, 32 KB) a stage, two units a stage for the others. Tensor memory: two accumulators of
+// 128 columns and the four operand slots of 64 fill the 512.
+__host__ __device__ constexpr int spl_gguf_stage_units(int rn) { return rn >= 128 ? 1 : 2; }
+// Stages of activations: four, or three where the widened blocks beside 64 or 128 rows leave no room for a fourth.
 __host__ __device__ constexpr int spl_gguf_bstages(int rn, int format) { return (rn >= 64 && format != SPL_GGUF_Q4K) ? 3 : 4; }
 #define SPL_GG_THREADS 480       // warps 0-3, 8-11 and 4-7: three dequant sets; 12 copies; 13-14 tensor-core issue
 __host__ __device__ constexpr size_t spl_gguf_smem_bytes(int rn, int format) {
-    return 1024 + size_t(SPL_GG_CSTAGES) * spl_gguf_pieces(format) * 2048 + size_t(spl_gguf_bstages(rn, format)) * SPL_TC_SUPER * rn * 128 + 1024;
+    return 1024 + size_t(SPL_GG_CSTAGES) * spl_gguf_pieces(format) * 2048 + size_t(spl_gguf_bstages(rn, format)) * spl_gguf_stage_units(rn) * 2 * rn * 128 + 1024;
 }
 __device__ __forceinline__ float spl_half_bits_to_float(uint32_t bits) { return __half2float(__ushort_as_half(uint16_t(bits))); }
 // Two fp32 values -> one register of two fp16, each rounded to nearest even.
@@ -196,32 +200,38 @@ __device__ __forceinline__ void spl_gguf_dequant64(const unsigned char *stage, i
     }
 }
 
-// Grid (tiles, splits, row blocks in use), as spl_gemm_q4_tc_kernel; `supers` super-blocks of 256 in the contraction,
-// `supers_per_split` of them a split.
+// Grid (tiles x row blocks in use, the row block the fast index; splits): the row blocks of a tile run together, so that a tile's weights
+// come from HBM once and from L2 for the others. `supers` super-blocks of 256 in the contraction, `supers_per_split` of them a split.
 template <int RN, int FMT>
 __global__ void __launch_bounds__(SPL_GG_THREADS, 1)
 spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfloat16 *__restrict__ act, float *out, int out_ld,
                         const float *residual, float *partials, int rows, int op_blocks, int supers_total, int supers_per_split, int *error_flag) {
-    constexpr int BST = spl_gguf_bstages(RN, FMT), CST = SPL_GG_CSTAGES, ASUP = 2, AST = 4 * ASUP, PIECES = spl_gguf_pieces(FMT);
-    constexpr int BTILE = SPL_TC_SUPER * RN * 128, WSTAGE = PIECES * 2048;
+    // A unit is two groups: what a dequant set converts at a time, an operand slot in tensor memory (AUN of them), a barrier of `done`.
+    constexpr int BST = spl_gguf_bstages(RN, FMT), CST = SPL_GG_CSTAGES, AUN = 4, PIECES = spl_gguf_pieces(FMT), SU = spl_gguf_stage_units(RN);
+    constexpr int BTILE = SU * 2 * RN * 128, WSTAGE = PIECES * 2048;
+    // done[un % 8]: the instructions that read unit un (its operand slot, its activations) have completed. Whoever waits for unit u asks
+    // while the barrier's next tenant, u + 8, cannot have completed: a converter at unit u + 4, the copier at the stage BST ahead.
+    static_assert(AUN < 8 && BST * SU <= 8, "a wait on `done` would meet the barrier's next tenant");
     extern __shared__ unsigned char spl_gg_smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(spl_gg_smem_raw) + 1023) & ~uintptr_t(1023));
-    unsigned char *b_ring = smem;                                   // [BST][4][RN * 128] activations
+    unsigned char *b_ring = smem;                                   // [BST][2 * SU][RN * 128] activations
     unsigned char *w_ring = b_ring + size_t(BST) * BTILE;           // [CST][pieces][128][16] blocks
     uint64_t *bars = reinterpret_cast<uint64_t *>(w_ring + size_t(CST) * WSTAGE);
-    uint64_t *full_c = bars, *empty_c = full_c + CST, *full_b = empty_c + CST, *empty_b = full_b + BST, *full_a = empty_b + BST, *finished = full_a + AST / 2;
+    uint64_t *full_c = bars, *empty_c = full_c + CST, *full_b = empty_c + CST, *done = full_b + BST, *full_a = done + 8, *finished = full_a + AUN;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(finished + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x, split = blockIdx.y, rb = blockIdx.z, row_blocks = op_blocks;
-    const int rows_padded = op_blocks * RN, groups = supers_total * SPL_TC_SUPER;
+    const int run_blocks = (rows + RN - 1) / RN, row_blocks = op_blocks;     // row blocks in use, and the operand's
+    const int tile = int(blockIdx.x) / run_blocks, rb = int(blockIdx.x) % run_blocks, split = blockIdx.y;
+    const int rows_padded = op_blocks * RN;
     const int s_first = split * supers_per_split, supers = min(supers_per_split, supers_total - s_first);
     const int units = supers * 2;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < CST; ++i) { spl_mbar_init(&full_c[i], 1); spl_mbar_init(&empty_c[i], 8); }
-        for (int i = 0; i < BST; ++i) { spl_mbar_init(&full_b[i], 1); spl_mbar_init(&empty_b[i], 2); }
-        for (int i = 0; i < AST / 2; ++i) spl_mbar_init(&full_a[i], 4);
+        for (int i = 0; i < BST; ++i) spl_mbar_init(&full_b[i], 1);
+        for (int i = 0; i < 8; ++i) spl_mbar_init(&done[i], 2);           // the commits of the two issuing warps
+        for (int i = 0; i < AUN; ++i) spl_mbar_init(&full_a[i], 4);
         spl_mbar_init(finished, 2);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -234,9 +244,8 @@ spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfl
     spl_tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     constexpr int NACC = RN <= 32 ? 4 : 2;
-    const uint32_t tmem_d = tmem, tmem_a = tmem + 128;
+    const uint32_t tmem_d = tmem, tmem_a = tmem + (NACC * RN > 128 ? NACC * RN : 128);
     bool ok = true;
-    (void)groups;
 
     if (!(warp == 12 && lane == 0)) spl_grid_begin();
     if (warp == 12) {
@@ -250,22 +259,28 @@ spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfl
             }
             spl_grid_begin();
             for (int j = 0; j < supers && ok; ++j) {
-                const int sc = j % CST, sbq = j % BST;
+                const int sc = j % CST;
                 if (j >= ahead) {
                     ok = spl_mbar_wait(&empty_c[sc], ((j / CST) & 1) ^ 1);
                     if (!ok) break;
                     spl_mbar_expect_tx(&full_c[sc], WSTAGE);
                     spl_bulk_g2s(w_ring + size_t(sc) * WSTAGE, wsrc + size_t(j) * WSTAGE, WSTAGE, &full_c[sc]);
                 }
-                ok = spl_mbar_wait(&empty_b[sbq], ((j / BST) & 1) ^ 1);
-                if (!ok) break;
-                spl_mbar_expect_tx(&full_b[sbq], uint32_t(BTILE));
-                if (row_blocks == 1) {
-                    spl_bulk_g2s(b_ring + size_t(sbq) * BTILE, bsrc + size_t(j) * BTILE, BTILE, &full_b[sbq]);
-                } else {
-                    for (int u = 0; u < SPL_TC_SUPER; ++u) {
-                        const size_t g = size_t(j) * SPL_TC_SUPER + u;
-                        spl_bulk_g2s(b_ring + size_t(sbq) * BTILE + u * RN * 128, bsrc + g * row_blocks * RN * 128, RN * 128, &full_b[sbq]);
+                for (int t = 0; t < 2 / SU && ok; ++t) {                  // the super-block's stages of activations
+                    const int stage = j * (2 / SU) + t, sbq = stage % BST;
+                    if (stage >= BST) {                                   // the last unit of the slot's last tenant: its warps' earlier ones have completed too
+                        const int u = (stage - BST) * SU + SU - 1;
+                        ok = spl_mbar_wait(&done[u & 7], (u >> 3) & 1);
+                        if (!ok) break;
+                    }
+                    spl_mbar_expect_tx(&full_b[sbq], uint32_t(BTILE));
+                    if (row_blocks == 1) {
+                        spl_bulk_g2s(b_ring + size_t(sbq) * BTILE, bsrc + size_t(stage) * BTILE, BTILE, &full_b[sbq]);
+                    } else {
+                        for (int u = 0; u < 2 * SU; ++u) {
+                            const size_t g = size_t(stage) * (2 * SU) + u;
+                            spl_bulk_g2s(b_ring + size_t(sbq) * BTILE + u * RN * 128, bsrc + g * row_blocks * RN * 128, RN * 128, &full_b[sbq]);
+                        }
                     }
                 }
             }
@@ -277,32 +292,31 @@ spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfl
         constexpr uint32_t idesc = spl_tc_idesc(RN);
         const uint64_t b_desc0 = spl_tc_desc_sw128(spl_smem_addr(b_ring));
         for (int j = 0; j < supers && ok; ++j) {
-            const int sbq = j % BST;
-            const uint64_t b_desc = b_desc0 + uint64_t((sbq * BTILE) >> 4);
-            const uint32_t a_base = tmem_a + (j % ASUP) * (SPL_TC_SUPER * 32);
-            ok = spl_mbar_wait_warp(&full_b[sbq], (j / BST) & 1);
-            if (!ok) break;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                const int un = 2 * j + half;
-                ok = spl_mbar_wait_warp(&full_a[un % (AST / 2)], (un / (AST / 2)) & 1);
+                const int un = 2 * j + half, stage = un / SU, sbq = stage % BST;
+                const uint64_t b_desc = b_desc0 + uint64_t((sbq * BTILE + (un % SU) * 2 * RN * 128) >> 4);
+                const uint32_t a_base = tmem_a + (un % AUN) * 64;
+                if (un % SU == 0) {
+                    ok = spl_mbar_wait_warp(&full_b[sbq], (stage / BST) & 1);
+                    if (!ok) break;
+                }
+                ok = spl_mbar_wait_warp(&full_a[un % AUN], (un / AUN) & 1);
                 if (!ok) break;
                 spl_tc_fence_after();
                 if (spl_elect_one()) {
 #pragma unroll
-                    for (int v = 0; v < 2; ++v) {
-                        const int u = 2 * half + v;
+                    for (int v = 0; v < 2; ++v)
 #pragma unroll
                         for (int l = 0; l < 2; ++l) {
                             const int ks = 2 * m + l, acc = NACC == 4 ? ks : m;
-                            const uint32_t d = tmem_d + acc * RN, a = a_base + u * 32 + ks * 8;
-                            const uint64_t b = b_desc + uint64_t((u * RN * 128 + ks * 32) >> 4);
+                            const uint32_t d = tmem_d + acc * RN, a = a_base + v * 32 + ks * 8;
+                            const uint64_t b = b_desc + uint64_t((v * RN * 128 + ks * 32) >> 4);
                             if (NACC == 2 && l > 0) spl_tc_mma_ts_acc(d, a, b, idesc);
-                            else if (j > 0 || u > 0) spl_tc_mma_ts_acc(d, a, b, idesc);
+                            else if (half > 0 || v > 0 || j > 0) spl_tc_mma_ts_acc(d, a, b, idesc);
                             else spl_tc_mma_ts(d, a, b, idesc, 0u);
                         }
-                    }
-                    if (half == 1) spl_tc_commit(&empty_b[sbq]);
+                    spl_tc_commit(&done[un & 7]);
                 }
                 __syncwarp();
             }
@@ -321,20 +335,20 @@ spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfl
             for (int v = 0; v < 2; ++v) spl_gguf_dequant64<FMT>(w_ring + size_t(sc) * WSTAGE, col, 2 * half + v, a[v]);
             __syncwarp();
             if (lane == 0) spl_mbar_arrive(&empty_c[sc]);
-            // The A slots were last used ASUP stages ago; that stage's completion is the one its activation stage is freed by.
-            if (j >= ASUP) ok = spl_mbar_wait(&empty_b[(j - ASUP) % BST], ((j - ASUP) / BST) & 1);
+            // The unit's slot was last used by unit un - AUN.
+            if (un >= AUN) ok = spl_mbar_wait(&done[(un - AUN) & 7], ((un - AUN) >> 3) & 1);
             if (!ok) break;
             spl_tc_fence_after();
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
-                const int sa = (j % ASUP) * SPL_TC_SUPER + 2 * half + v;
+                const int sa = (un % AUN) * 2 + v;
                 spl_tc_st16(tmem_a + lane_base + sa * 32, *reinterpret_cast<uint32_t (*)[16]>(&a[v][0]));
                 spl_tc_st16(tmem_a + lane_base + sa * 32 + 16, *reinterpret_cast<uint32_t (*)[16]>(&a[v][16]));
             }
             spl_tc_st_wait();
             spl_tc_fence_before();
             __syncwarp();
-            if (lane == 0) spl_mbar_arrive(&full_a[un % (AST / 2)]);
+            if (lane == 0) spl_mbar_arrive(&full_a[un % AUN]);
         }
         if (ok) ok = spl_mbar_wait(finished, 0);
         if (ok) {

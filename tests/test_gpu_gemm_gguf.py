@@ -54,3 +54,13 @@ def test_27b_inner_dimensions_and_split_contraction(kind, n, k):
     rng = np.random.default_rng(2)
     w = rng.normal(0, 0.02, (n, k)).astype(np.float32)
     check(kind, O.quantize_gguf(kind, w), 64, seed=9, residual=False)
+
+
+@pytest.mark.parametrize("kind", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("rows,n,k", [(65, 200, 256), (127, 384, 512), (128, 130, 1024), (129, 256, 2560), (200, 640, 3072), (385, 128, 768)])
+def test_blocks_of_128_rows(kind, rows, n, k):
+    """Steps of more than 64 rows: one to four row blocks with ragged ends, contractions of one super-block to twelve (fewer and more units than the
+    rings hold), cut and whole, with the residual."""
+    rng = np.random.default_rng(rows)
+    w = rng.normal(0, 0.02, (n, k)).astype(np.float32)
+    check(kind, O.quantize_gguf(kind, w), rows, seed=k)
