@@ -406,7 +406,9 @@ void launch_gemm_gguf_tc(cudaStream_t stream, const SplGgufDev &w, const GemmOpe
     const int supers = w.k / 256;
     const int row_blocks = (rows + RN - 1) / RN, rows_padded = op.blocks * RN;
     // The q4 rule in units of four groups: a split is a whole number of super-blocks.
-    const int splits4 = choose_splits(w.tiles * row_blocks, supers * 4, 148, partial_floats, size_t(rows_padded) * w.ld);
+    // The 128-row block keeps the cut that blocks of 64 rows would have: the order of a sum, and so the output to the bit, is a function of the tensor and the
+    // row count alone.
+    const int splits4 = choose_splits(w.tiles * ((rows + std::min(RN, 64) - 1) / std::min(RN, 64)), supers * 4, 148, partial_floats, size_t(rows_padded) * w.ld);
     const int sps = (supers + splits4 - 1) / splits4, splits = (supers + sps - 1) / sps;
     const size_t smem = spl_gguf_smem_bytes(RN, FMT);
     launch_step(spl_gemm_gguf_tc_kernel<RN, FMT>, dim3(w.tiles * row_blocks, splits), dim3(SPL_GG_THREADS), smem, stream,
