@@ -616,7 +616,7 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
             profile_end(e);
             ggemm(L.g_gate_up, gxn, e->gate_up, nullptr, live);
             profile_begin(e, KLASS_ELEMENTWISE, 0);
-            launch_step(spl_swiglu_kernel, dim3(g.inter / 64, live), dim3(32), 0, e->stream, (const float *)e->gate_up, e->gate_up_ld, g.inter, act);
+            launch_step(spl_swiglu_kernel, dim3((g.inter / 64 + 7) / 8, live), dim3(256), 0, e->stream, (const float *)e->gate_up, e->gate_up_ld, g.inter, act);
             profile_end(e);
             ggemm(L.g_down, gact, e->h, e->h, live);
         } else if (live > 0) {

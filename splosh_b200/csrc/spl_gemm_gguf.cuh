@@ -433,10 +433,12 @@ __global__ void spl_embed_gguf_kernel(const unsigned char *__restrict__ table, i
 }
 
 // act = bf16(silu(gate) * up) of an unfused gate|up output [rows][2 inter] (gate columns first) as the down projection's
-// operand with its per-64 sums (Sources/Shaders/engine.metal:200-219). Grid (inter / 64, rows), 32 threads.
-__global__ void spl_swiglu_kernel(const float *__restrict__ gate_up, int ld, int inter, SplOperand out) {
+// operand with its per-64 sums (Sources/Shaders/engine.metal:200-219). Grid (groups of 64 in eights, rows), 256 threads: a warp a group (a block of
+// one warp each is 54,400 blocks for a 200-row prompt of the 27B shape, and what that costs is their launch).
+__global__ void __launch_bounds__(256) spl_swiglu_kernel(const float *__restrict__ gate_up, int ld, int inter, SplOperand out) {
     spl_grid_begin();
-    const int group = blockIdx.x, row = blockIdx.y, lane = threadIdx.x, n = group * 64 + 2 * lane;
+    const int group = blockIdx.x * 8 + (threadIdx.x >> 5), row = blockIdx.y, lane = threadIdx.x & 31, n = group * 64 + 2 * lane;
+    if (group * 64 >= inter) return;
     const float2 g = *reinterpret_cast<const float2 *>(gate_up + size_t(row) * ld + n), u = *reinterpret_cast<const float2 *>(gate_up + size_t(row) * ld + inter + n);
     const float v0 = spl_bf16_to_float(spl_float_to_bf16(spl_silu_exact(g.x) * u.x)), v1 = spl_bf16_to_float(spl_float_to_bf16(spl_silu_exact(g.y) * u.y));
     *reinterpret_cast<__half2 *>(reinterpret_cast<__half *>(out.values) + out.at(row, n)) = __halves2half2(__float2half_rn(v0), __float2half_rn(v1));
