@@ -648,6 +648,8 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
     }
     if (!fits) return e->fail(SPL_ERR_INVALID_ROWS, "invalid step rows: the GEMM scratch is smaller than the step needs");
     SPL_CUDA(cudaEventRecord(e->ev_end, e->stream));
+    // The error words ride home with the step, behind its tables' pinned words: a copy of their own after the wait costs the host a second trip.
+    SPL_CUDA(cudaMemcpyAsync(e->tables_host + e->tables_words, e->tc_error, 4 * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     e->flying_rows = R; e->flying_logit_rows = int(t->logit_rows);
     return check_launch(e, "step launch");
 }
@@ -657,8 +659,8 @@ spl_status finish_step(spl_engine *e, spl_step_stats *stats) {
     SPL_CUDA(cudaSetDevice(e->device));
     SPL_CUDA(cudaStreamSynchronize(e->stream));
     {
-        int flag[4] = {0, 0, 0, 0};
-        SPL_CUDA(cudaMemcpy(flag, e->tc_error, sizeof flag, cudaMemcpyDeviceToHost));
+        int flag[4];
+        std::memcpy(flag, e->tables_host + e->tables_words, sizeof flag);
         if (flag[0]) {
             cudaMemset(e->tc_error, 0, sizeof flag);
             if (flag[0] >= 100) return e->fail(SPL_ERR_TIMEOUT, "an attention scan block gave up waiting (warp " + std::to_string(flag[0] - 100) + ")");
@@ -888,7 +890,7 @@ spl_status create(const spl_geometry *gp, const spl_config *cp, spl_engine *e) {
     if ((s = device_alloc(e, &e->attn_partials, e->attn_partial_floats, &e->scratch_bytes)) != SPL_OK) return s;
     e->tables_words = size_t(R) * 5 + size_t(e->c.max_slots) * 5 + size_t(LR) + size_t(R) * 2 + size_t(e->c.max_slots) * e->host->max_pages + 64
                       + size_t(e->c.max_slots) * 4 + (size_t(R) / SPL_GDN_CHUNK + e->c.max_slots) * 4 + 16;
-    SPL_CUDA(cudaMallocHost(reinterpret_cast<void **>(&e->tables_host), e->tables_words * 4));
+    SPL_CUDA(cudaMallocHost(reinterpret_cast<void **>(&e->tables_host), (e->tables_words + 4) * 4));      // and four words for the step's error words
     if ((s = device_alloc(e, &e->tables_dev, e->tables_words)) != SPL_OK) return s;
     SPL_CUDA(cudaStreamSynchronize(e->stream));
     return SPL_OK;
