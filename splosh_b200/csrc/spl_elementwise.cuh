@@ -135,7 +135,8 @@ spl_argmax_kernel(const float *__restrict__ logits, int ld, int limit, int32_t *
 // times: two warp-wide reductions find the best key and its lowest index, and the lane that held it looks for its next
 // best in one group. A block merges its eight sorted lists; the second kernel merges a row's blocks the same way, a lane a
 // list. Bound: the row's one trip from HBM for many rows, the chain of k picks for few.
-// One block a row scanning it k times (what this replaced) took 1.31-1.34 ms for k = 20 of 248,077 at 12 to 64 rows.
+// One block a row scanning it k times (what this replaced) took 1.31-1.34 ms for k = 20 of 248,077 at 12 to 64 rows; a
+// twelve-row decode step with its top-k went from 9.07 to 7.76 ms.
 //
 // A key is the float's bits made to order as unsigned numbers, minus zero taken as zero (the two are equal values, so the lower
 // index goes first); 0 stands for what is never picked: NaN, -inf and what lies past the limit.
