@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -400,37 +401,61 @@ bool launch_gemm_rows(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand 
     return launch_gemm_tc<128>(stream, w, op, out, residual, rows, scratch, x, launches);
 }
 
-template <int RN, int FMT>
-void launch_gemm_gguf_tc(cudaStream_t stream, const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows,
-                         float *partials, size_t partial_floats, int *error_flag) {
+// Where a cut GGUF GEMM's blocks leave their partial sums, the launch's error words, the device's SM count.
+struct GgufScratch { float *partials; size_t floats; int *error_flag; int sms; };
+
+// The pieces of a GGUF tensor's contraction for `rows` rows: the q4 rule in units of four groups, a piece a whole number of super-blocks. Blocks
+// of 64 and of 128 rows are cut alike, as suits blocks of 64, and both keep two accumulators: the order of a sum, and so the output to the
+// bit, does not depend on which of the two a step takes (unless the scratch's cap binds: it sees the rows padded to the block). What that
+// leaves: 200 rows on 5,120 x 17,408 are cut in 4, where by the rule's own count the launched grid would be better off with 3 (224 against 264).
+int gguf_pieces(const SplGgufDev &w, int rows, int rows_padded, const GgufScratch &scratch) {
     const int supers = w.k / 256;
-    const int row_blocks = (rows + RN - 1) / RN, rows_padded = op.blocks * RN;
-    // The q4 rule in units of four groups: a split is a whole number of super-blocks.
-    // The 128-row block keeps the cut that blocks of 64 rows would have: the order of a sum, and so the output to the bit, is a function of the tensor and the
-    // row count alone.
-    const int splits4 = choose_splits(w.tiles * ((rows + std::min(RN, 64) - 1) / std::min(RN, 64)), supers * 4, 148, partial_floats, size_t(rows_padded) * w.ld);
-    const int sps = (supers + splits4 - 1) / splits4, splits = (supers + sps - 1) / sps;
+    const int splits = choose_splits(w.tiles * ((rows + 63) / 64), supers * 4, scratch.sms, scratch.floats, size_t(rows_padded) * w.ld);
+    const int per = (supers + splits - 1) / splits;
+    return (supers + per - 1) / per;
+}
+// Rows a block of the operand that `readers` read, in a step of `rows` rows. A weight is formed once a block, so a block of 128 rows converts
+// half of what two of 64 do; but it takes longer than one of 64 (128 columns an instruction, a shorter ring of activations): 1.24, 1.40 and 1.52
+// times for Q4_K, Q5_K and Q6_K (5,120 x 17,408 at 129 rows, 80 blocks of 128 or 120 of 64, one wave on 148 SMs either way: 82.0 -> 101.8,
+// 84.2 -> 118.0, 80.8 -> 123.1 us). So 128 is taken where it saves more than that in waves of blocks over the readers' launches. Measured at 200 rows,
+// 34,816 x 5,120 (8 waves or 4): 184 -> 121, 189 -> 140, 181 -> 143 us; at 129 rows (6 or 4): 141 -> 119, 145 -> 137, 139 -> 141 us.
+int gguf_operand_rn(int rows, std::initializer_list<const SplGgufDev *> readers, const GgufScratch &scratch) {
+    if (rows <= 64) return operand_rn(rows);
+    double cost[2] = {0, 0};
+    for (const SplGgufDev *w : readers) {
+        const double wide = w->format == SPL_GGUF_Q4K ? 1.25 : w->format == SPL_GGUF_Q5K ? 1.40 : 1.52;
+        for (int i = 0; i < 2; ++i) {
+            const int rn = 64 << i, blocks = (rows + rn - 1) / rn, pieces = gguf_pieces(*w, rows, blocks * rn, scratch);
+            const int waves = (w->tiles * blocks * pieces + scratch.sms - 1) / scratch.sms, supers = w->k / 256;
+            cost[i] += double(waves) * ((supers + pieces - 1) / pieces) * (i ? wide : 1.0);
+        }
+    }
+    return cost[1] < cost[0] ? 128 : 64;
+}
+
+template <int RN, int FMT>
+void launch_gemm_gguf_tc(cudaStream_t stream, const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows, const GgufScratch &scratch) {
+    const int supers = w.k / 256, row_blocks = (rows + RN - 1) / RN, rows_padded = op.blocks * RN;
+    const int splits = gguf_pieces(w, rows, rows_padded, scratch), sps = (supers + splits - 1) / splits;
     const size_t smem = spl_gguf_smem_bytes(RN, FMT);
     launch_step(spl_gemm_gguf_tc_kernel<RN, FMT>, dim3(w.tiles * row_blocks, splits), dim3(SPL_GG_THREADS), smem, stream,
-                w.blocks, op.values, out, w.ld, residual, partials, rows, op.blocks, supers, sps, error_flag);
+                w.blocks, op.values, out, w.ld, residual, scratch.partials, rows, op.blocks, supers, sps, scratch.error_flag);
     if (splits > 1) {
         const size_t total = size_t(rows) * w.ld / 4;
-        launch_step(spl_gemm_reduce_kernel, dim3(int(std::min<size_t>((total + 255) / 256, 2048))), dim3(256), 0, stream, partials, splits, rows_padded, rows, w.ld, residual, out);
+        launch_step(spl_gemm_reduce_kernel, dim3(int(std::min<size_t>((total + 255) / 256, 2048))), dim3(256), 0, stream, scratch.partials, splits, rows_padded, rows, w.ld, residual, out);
     }
 }
 template <int FMT>
-void launch_gemm_gguf_rows(cudaStream_t stream, const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows,
-                           float *partials, size_t partial_floats, int *error_flag) {
-    if (op.rn == 16) launch_gemm_gguf_tc<16, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
-    else if (op.rn == 32) launch_gemm_gguf_tc<32, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
-    else if (op.rn == 64) launch_gemm_gguf_tc<64, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
-    else launch_gemm_gguf_tc<128, FMT>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
+void launch_gemm_gguf_rows(cudaStream_t stream, const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows, const GgufScratch &scratch) {
+    if (op.rn == 16) launch_gemm_gguf_tc<16, FMT>(stream, w, op, out, residual, rows, scratch);
+    else if (op.rn == 32) launch_gemm_gguf_tc<32, FMT>(stream, w, op, out, residual, rows, scratch);
+    else if (op.rn == 64) launch_gemm_gguf_tc<64, FMT>(stream, w, op, out, residual, rows, scratch);
+    else launch_gemm_gguf_tc<128, FMT>(stream, w, op, out, residual, rows, scratch);
 }
-void launch_gemm_gguf(cudaStream_t stream, const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows,
-                      float *partials, size_t partial_floats, int *error_flag) {
-    if (w.format == SPL_GGUF_Q6K) launch_gemm_gguf_rows<SPL_GGUF_Q6K>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
-    else if (w.format == SPL_GGUF_Q5K) launch_gemm_gguf_rows<SPL_GGUF_Q5K>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
-    else launch_gemm_gguf_rows<SPL_GGUF_Q4K>(stream, w, op, out, residual, rows, partials, partial_floats, error_flag);
+void launch_gemm_gguf(cudaStream_t stream, const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows, const GgufScratch &scratch) {
+    if (w.format == SPL_GGUF_Q6K) launch_gemm_gguf_rows<SPL_GGUF_Q6K>(stream, w, op, out, residual, rows, scratch);
+    else if (w.format == SPL_GGUF_Q5K) launch_gemm_gguf_rows<SPL_GGUF_Q5K>(stream, w, op, out, residual, rows, scratch);
+    else launch_gemm_gguf_rows<SPL_GGUF_Q4K>(stream, w, op, out, residual, rows, scratch);
 }
 
 bool launch_gemm(spl_engine *e, const SplQ4Dev &w, const GemmOperand &op, float *out, const float *residual, int rows, const GemmExtras &x = GemmExtras()) {
@@ -513,9 +538,14 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
 
     const int H = g.hidden;
     // GEMM operands of this step: row blocks of rn rows, in the tile layout the tensor cores read.
-    const int rn = operand_rn(R), blocks = (R + rn - 1) / rn;
-    const SplOperand xn{e->xn, e->xn_sums, rn, blocks}, core{e->core, e->core_sums, rn, blocks}, act{e->act, e->act_sums, rn, blocks};
-    const GemmOperand gxn{e->xn, e->xn_sums, rn, blocks}, gcore{e->core, e->core_sums, rn, blocks}, gact{e->act, e->act_sums, rn, blocks};
+    // (The blocks of a model have two shapes: its first gated-delta block and its first attention block stand for them.)
+    const GgufScratch gscratch{e->partials, e->partial_floats, e->tc_error, e->sms};
+    const LayerWeights &first = e->layers[0], &fourth = e->layers[std::min<size_t>(3, e->layers.size() - 1)];
+    const int rn = gguf ? gguf_operand_rn(R, {&first.g_in_proj, &fourth.g_in_proj, &first.g_gate_up}, gscratch) : operand_rn(R), blocks = (R + rn - 1) / rn;
+    const int core_rn = gguf ? gguf_operand_rn(R, {&first.g_out_proj, &fourth.g_out_proj}, gscratch) : rn, core_blocks = (R + core_rn - 1) / core_rn;
+    const int act_rn = gguf ? gguf_operand_rn(R, {&first.g_down}, gscratch) : rn, act_blocks = (R + act_rn - 1) / act_rn;
+    const SplOperand xn{e->xn, e->xn_sums, rn, blocks}, core{e->core, e->core_sums, core_rn, core_blocks}, act{e->act, e->act_sums, act_rn, act_blocks};
+    const GemmOperand gxn{e->xn, e->xn_sums, rn, blocks}, gcore{e->core, e->core_sums, core_rn, core_blocks}, gact{e->act, e->act_sums, act_rn, act_blocks};
     profile_begin(e, KLASS_ELEMENTWISE, 0);
     if (gguf) launch_step(spl_embed_gguf_kernel, dim3(R), dim3(256), 0, e->stream, (const unsigned char *)e->g_embed, e->g_embed_format, (const uint32_t *)e->d_tokens, e->h, H);
     else launch_step(spl_embed_q4_kernel, dim3(R), dim3(128), 0, e->stream, e->embed_packed, e->embed_scales, e->embed_biases, e->d_tokens, e->h, H);
@@ -524,7 +554,7 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
     // unfused SiLU gate (the results are the deferred forms' up to the operand's rounding point).
     auto ggemm = [&](const SplGgufDev &w, const GemmOperand &op, float *out, const float *residual, int rows) {
         profile_begin(e, KLASS_GEMM, double(w.bytes()) * ((rows + op.rn - 1) / op.rn));
-        launch_gemm_gguf(e->stream, w, op, out, residual, rows, e->partials, e->partial_floats, e->tc_error);
+        launch_gemm_gguf(e->stream, w, op, out, residual, rows, gscratch);
         profile_end(e);
     };
 
@@ -640,7 +670,7 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
     }
     if (t->logit_rows > 0) {
         profile_begin(e, KLASS_OTHER, 0);
-        const int lrn = operand_rn(int(t->logit_rows)), lblocks = (int(t->logit_rows) + lrn - 1) / lrn;
+        const int lrn = gguf ? gguf_operand_rn(int(t->logit_rows), {&e->g_head}, gscratch) : operand_rn(int(t->logit_rows)), lblocks = (int(t->logit_rows) + lrn - 1) / lrn;
         norm(int(t->logit_rows), e->final_norm, e->d_gather, SplOperand{e->hsn, e->hsn_sums, lrn, lblocks});
         profile_end(e);
         if (gguf) ggemm(e->g_head, GemmOperand{e->hsn, e->hsn_sums, lrn, lblocks}, e->logits, nullptr, int(t->logit_rows));
@@ -1399,6 +1429,17 @@ spl_status spl_debug_pair_blocks(spl_engine *, int32_t enabled) {
     return SPL_OK;
 }
 
+spl_status spl_debug_gguf_plan(int32_t format, int32_t n, int32_t k, int32_t rows, int32_t sms, int32_t *block_rows, int32_t *pieces) {
+    if (n <= 0 || k <= 0 || k % 256 || rows <= 0 || sms <= 0 || !block_rows || !pieces ||
+        (format != SPL_GGUF_Q4K && format != SPL_GGUF_Q5K && format != SPL_GGUF_Q6K)) return SPL_ERR_INVALID_ARGUMENT;
+    SplGgufDev w;
+    w.n = n; w.ld = round16(n); w.tiles = (n + 127) / 128; w.k = k; w.format = format;
+    const GgufScratch scratch{nullptr, SIZE_MAX, nullptr, sms};
+    *block_rows = gguf_operand_rn(rows, {&w}, scratch);
+    *pieces = gguf_pieces(w, rows, (rows + *block_rows - 1) / *block_rows * *block_rows, scratch);
+    return SPL_OK;
+}
+
 spl_status spl_debug_gdn_chunk_min(spl_engine *e, int32_t rows) {
     if (!e || rows < SPL_GDN_CHUNK) return SPL_ERR_INVALID_ARGUMENT;
     e->gdn_chunk_min = rows;
@@ -1842,9 +1883,9 @@ spl_status spl_op_gemm_gguf(int32_t device, int32_t format, const uint8_t *block
     SPL_CUDA(cudaStreamCreate(&e->stream));
     SplGgufDev w;
     w.n = n; w.ld = round16(n); w.tiles = (n + 127) / 128; w.k = k; w.format = format;
-    const int ld = w.ld, rn = operand_rn(rows), row_blocks = (rows + rn - 1) / rn;
+    const int ld = w.ld;
+    const int rn = gguf_operand_rn(rows, {&w}, GgufScratch{nullptr, size_t(16) * ((rows + 127) / 128 * 128) * ld, nullptr, e->sms}), row_blocks = (rows + rn - 1) / rn;
     float *d_act32 = nullptr, *d_out = nullptr, *d_sums = nullptr; __nv_bfloat16 *d_act = nullptr; int *d_flag = nullptr; unsigned char *d_native = nullptr;
-    e->partial_floats = size_t(16) * row_blocks * rn * ld;
     spl_status s = SPL_OK;
     if (cudaMalloc(reinterpret_cast<void **>(&w.blocks), w.device_bytes()) != cudaSuccess || cudaMalloc(reinterpret_cast<void **>(&d_native), w.bytes()) != cudaSuccess)
         s = SPL_ERR_ALLOCATION_FAILED;
@@ -1853,6 +1894,7 @@ spl_status spl_op_gemm_gguf(int32_t device, int32_t format, const uint8_t *block
     if (s == SPL_OK) s = device_alloc(e, &d_sums, spl_operand_sums_floats(size_t(row_blocks) * rn, k));
     if (s == SPL_OK) s = device_alloc(e, &d_out, size_t(rows) * ld);
     if (s == SPL_OK) s = device_alloc(e, &d_flag, 64);
+    e->partial_floats = size_t(16) * row_blocks * rn * ld;
     if (s == SPL_OK) s = device_alloc(e, &e->partials, e->partial_floats);
     if (s == SPL_OK) {
         cudaMemsetAsync(w.blocks, 0, w.device_bytes(), e->stream);           // columns past n are zero blocks: weights 0
@@ -1865,7 +1907,7 @@ spl_status spl_op_gemm_gguf(int32_t device, int32_t format, const uint8_t *block
         cudaMemcpyAsync(d_act32, activations, size_t(rows) * k * 4, cudaMemcpyHostToDevice, e->stream);
         spl_operand_kernel<<<rows, 256, 0, e->stream>>>(d_act32, SplOperand{d_act, d_sums, rn, row_blocks}, k);
         if (residual) cudaMemcpy2DAsync(d_out, size_t(ld) * 4, residual, size_t(n) * 4, size_t(n) * 4, rows, cudaMemcpyHostToDevice, e->stream);
-        launch_gemm_gguf(e->stream, w, GemmOperand{d_act, d_sums, rn, row_blocks}, d_out, residual ? d_out : nullptr, rows, e->partials, e->partial_floats, d_flag);
+        launch_gemm_gguf(e->stream, w, GemmOperand{d_act, d_sums, rn, row_blocks}, d_out, residual ? d_out : nullptr, rows, GgufScratch{e->partials, e->partial_floats, d_flag, e->sms});
         s = check_launch(e, "gguf gemm");
         if (cudaStreamSynchronize(e->stream) != cudaSuccess) s = SPL_ERR_DEVICE;
         int flag = 0;

@@ -85,7 +85,7 @@ __global__ void spl_repack_gguf_kernel(const unsigned char *__restrict__ native,
 // the coming phase would be answered by the one before: the set would read the old tenant and hand its slot back early
 // (at two stages, 64 rows of the byte-wide types: a wrong sum, or a launch failure in the blocks after it).
 #define SPL_GG_CSTAGES 3
-// The 128-row block (steps of more than 64 rows: prompt chunks) forms a weight once for twice the rows of the 64-row block. Its
+// The 128-row block (steps of more than 64 rows, where it saves waves of blocks) forms a weight once for twice the rows of the 64-row block. Its
 // activations come a unit (two groups, 32 KB) a stage, two units a stage for the others. Tensor memory: two accumulators of
 // 128 columns and the four operand slots of 64 fill the 512. A step with a 200-row Q4_K prompt of the 27B shape: 46.2 -> 33.7 ms (of it the SiLU
 // kernel's larger blocks and the top-k).

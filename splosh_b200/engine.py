@@ -211,6 +211,7 @@ def lib():
             "spl_debug_taps": (i32, [vp, i32]),
             "spl_debug_kv_store": (i32, [vp, i32]),
             "spl_debug_gdn_chunk_min": (i32, [vp, i32]),
+            "spl_debug_gguf_plan": (i32, [i32, i32, i32, i32, i32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
             "spl_debug_pair_blocks": (i32, [vp, i32]),
             "spl_debug_wait_budget": (i32, [vp, C.c_int64]),
             "spl_debug_drop_weight_stage": (i32, [vp, i32]),
@@ -741,6 +742,15 @@ RESIDENT = ["in_proj", "out_proj", "gate_up", "down", "head"]
 def debug_pair_blocks(enabled=True):
     """Steps of more than 64 rows on the pair form of the 128-row GEMM block (default) or on the one-tile block (process-wide)."""
     lib().spl_debug_pair_blocks(None, int(enabled))
+
+
+def debug_gguf_plan(kind, n, k, rows, sms=148):
+    """(rows a block, pieces of the contraction) of a GGUF GEMM's launch; no device needed."""
+    block_rows, pieces = C.c_int32(0), C.c_int32(0)
+    status = lib().spl_debug_gguf_plan(GGUF_TYPE[kind], n, k, rows, sms, C.byref(block_rows), C.byref(pieces))
+    if status:
+        raise EngineError(status, "spl_debug_gguf_plan refused its arguments")
+    return block_rows.value, pieces.value
 
 
 def splw_check(path):

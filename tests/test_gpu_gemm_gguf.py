@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 import splosh_b200 as S
+from splosh_b200.engine import debug_gguf_plan
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -57,10 +58,14 @@ def test_27b_inner_dimensions_and_split_contraction(kind, n, k):
 
 
 @pytest.mark.parametrize("kind", ["Q4_K", "Q5_K", "Q6_K"])
-@pytest.mark.parametrize("rows,n,k", [(65, 200, 256), (127, 384, 512), (128, 130, 1024), (129, 256, 2560), (200, 640, 3072), (385, 128, 768)])
-def test_blocks_of_128_rows(kind, rows, n, k):
-    """Steps of more than 64 rows: one to four row blocks with ragged ends, contractions of one super-block to twelve (fewer and more units than the
-    rings hold), cut and whole, with the residual."""
+@pytest.mark.parametrize("rows,n,k,block,pieces", [
+    (65, 200, 256, 64, 1), (127, 384, 512, 64, 1), (128, 130, 1024, 64, 2), (129, 256, 2560, 64, 5), (200, 640, 3072, 64, 6), (385, 128, 768, 64, 1),
+    (65, 12800, 256, 128, 1), (127, 18810, 512, 128, 1), (128, 12850, 1024, 128, 1), (193, 9450, 2560, 128, 1), (200, 5120, 3072, 128, 1), (385, 3200, 768, 128, 1),
+    (65, 5120, 6144, 128, 3)])
+def test_several_row_blocks(kind, rows, n, k, block, pieces):
+    """Steps of more than 64 rows: one to seven row blocks with ragged ends in blocks of 64 rows (few tiles) and of 128 (where they save a wave),
+    contractions of one super-block to 24 (fewer and more units than the rings hold), cut and whole, with the residual."""
+    assert debug_gguf_plan(kind, n, k, rows) == (block, pieces)
     rng = np.random.default_rng(rows)
     w = rng.normal(0, 0.02, (n, k)).astype(np.float32)
     check(kind, O.quantize_gguf(kind, w), rows, seed=k)
