@@ -143,6 +143,8 @@ spl_argmax_kernel(const float *__restrict__ logits, int ld, int limit, int32_t *
 #define SPL_TOPK_WARP 1024               // values of a warp
 #define SPL_TOPK_STRETCH (8 * SPL_TOPK_WARP)
 #define SPL_TOPK_MAX 64
+// Floats of device scratch a top-k takes at most: the rows' lists and their picks (ids, then values).
+inline size_t spl_topk_floats(int rows, int vocab) { return size_t(rows) * (size_t(vocab + SPL_TOPK_STRETCH - 1) / SPL_TOPK_STRETCH + 1) * SPL_TOPK_MAX * 2; }
 __device__ __forceinline__ uint32_t spl_topk_key(float v) {
     if (!(v > -INFINITY)) return 0u;
     const uint32_t b = __float_as_uint(v + 0.0f);

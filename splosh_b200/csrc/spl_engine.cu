@@ -81,7 +81,7 @@ struct spl_engine {
     // Drafter feature taps (Engine.swift:330-331, 1488-1497): the residual stream after the listed blocks, [row][tap][hidden].
     float *features = nullptr;
     std::vector<int> feature_layers;
-    uint2 *topk_lists = nullptr; int32_t *topk_picks = nullptr, *topk_host = nullptr;      // allocated by the first spl_topk
+    int32_t *topk_host = nullptr;      // pinned, allocated by the first spl_topk (its device side is in `partials`, which no kernel uses between steps)
     __half *q = nullptr;
     int32_t *argmax_ids = nullptr;
     int proj_ld = 0, gate_up_ld = 0, core_ld = 0, logits_ld = 0;
@@ -894,7 +894,7 @@ spl_status create(const spl_geometry *gp, const spl_config *cp, spl_engine *e) {
     if ((s = device_alloc(e, &e->logits, size_t(LR) * e->logits_ld, &e->scratch_bytes)) != SPL_OK) return s;
     if ((s = device_alloc(e, &e->argmax_ids, size_t(LR), &e->scratch_bytes)) != SPL_OK) return s;
     e->partial_floats = size_t(16) * RP * std::max(H, 4096);      // split-K partial sums of the GGUF kernel
-    if ((s = device_alloc(e, &e->partials, e->partial_floats, &e->scratch_bytes)) != SPL_OK) return s;
+    if ((s = device_alloc(e, &e->partials, std::max(e->partial_floats, spl_topk_floats(LR, g.vocab)), &e->scratch_bytes)) != SPL_OK) return s;
     // Where the blocks of a cut tile of the q4 GEMM leave their partial sums: a slot of rn x 128 sums a block.
     const int row_blocks = std::max(RP, LP) / 128;      // more than 64 rows go in blocks of 128
     // The most slot space any of the engine's tensors takes, at any row count.
@@ -955,7 +955,7 @@ void spl_engine_destroy(spl_engine *e) {
     for (auto p : e->state) cudaFree(p); for (auto p : e->conv) cudaFree(p); for (auto p : e->journal) cudaFree(p);
     cudaFree(e->h); cudaFree(e->xn); cudaFree(e->proj); cudaFree(e->gdn_act); cudaFree(e->core); cudaFree(e->gate_up); cudaFree(e->act);
     cudaFree(e->q); cudaFree(e->hsn); cudaFree(e->logits); cudaFree(e->argmax_ids); cudaFree(e->partials); cudaFree(e->attn_partials);
-    cudaFree(e->taps); cudaFree(e->features); cudaFree(e->topk_lists); cudaFree(e->topk_picks); cudaFreeHost(e->topk_host); cudaFree(e->tables_dev); cudaFree(e->gdn_records); cudaFree(e->gdn_o_raw); cudaFree(e->slots); cudaFree(e->xn_squares); cudaFree(e->xn_sums); cudaFree(e->core_sums); cudaFree(e->act_sums); cudaFree(e->hsn_sums); cudaFree(e->tc_error);
+    cudaFree(e->taps); cudaFree(e->features); cudaFreeHost(e->topk_host); cudaFree(e->tables_dev); cudaFree(e->gdn_records); cudaFree(e->gdn_o_raw); cudaFree(e->slots); cudaFree(e->xn_squares); cudaFree(e->xn_sums); cudaFree(e->core_sums); cudaFree(e->act_sums); cudaFree(e->hsn_sums); cudaFree(e->tc_error);
     if (e->tables_host) cudaFreeHost(e->tables_host);
     for (ProfileSlot &s : e->profile_slots) { cudaEventDestroy(s.begin); cudaEventDestroy(s.end); }
     if (e->ev_begin) cudaEventDestroy(e->ev_begin);
@@ -1286,20 +1286,19 @@ spl_status spl_topk(spl_engine *e, int32_t vocab_limit, int32_t k, int32_t *ids,
     SPL_NOT_IN_FLIGHT(e);
     if (e->last_logit_rows == 0) return SPL_OK;
     SPL_CUDA(cudaSetDevice(e->device));
-    // Room for every logit row at the largest k: the rows' candidate lists, and the picks (ids, then values) with a pinned copy.
-    const size_t max_rows = size_t(e->host->config.max_logit_rows), max_stretches = size_t(e->g.vocab + SPL_TOPK_STRETCH - 1) / SPL_TOPK_STRETCH;
-    if (!e->topk_lists) SPL_CUDA(cudaMalloc(reinterpret_cast<void **>(&e->topk_lists), max_rows * max_stretches * SPL_TOPK_MAX * sizeof(uint2)));
-    if (!e->topk_picks) SPL_CUDA(cudaMalloc(reinterpret_cast<void **>(&e->topk_picks), max_rows * SPL_TOPK_MAX * 8));
+    const size_t max_rows = size_t(e->host->config.max_logit_rows);
     if (!e->topk_host) SPL_CUDA(cudaMallocHost(reinterpret_cast<void **>(&e->topk_host), max_rows * SPL_TOPK_MAX * 8));
     const int rows = e->last_logit_rows, stretches = (vocab_limit + SPL_TOPK_STRETCH - 1) / SPL_TOPK_STRETCH;
     const size_t picks = size_t(rows) * k, staged_bytes = size_t(stretches) * k * sizeof(uint2) + stretches;
     const bool staged = staged_bytes <= 48 * 1024;
-    launch_step(spl_topk_stretch_kernel, dim3(stretches, rows), dim3(256), 0, e->stream, (const float *)e->logits, e->logits_ld, vocab_limit, k, e->topk_lists);
-    launch_step(spl_topk_merge_kernel, dim3(rows), dim3(32), staged ? staged_bytes : size_t(stretches), e->stream, (const float *)e->logits, e->logits_ld, (const uint2 *)e->topk_lists,
-                stretches, k, staged ? 1 : 0, e->topk_picks, reinterpret_cast<float *>(e->topk_picks) + picks);
+    int32_t *ids_dev = reinterpret_cast<int32_t *>(e->partials);      // the picks: ids, then values; behind them the rows' lists
+    uint2 *lists = reinterpret_cast<uint2 *>(e->partials) + picks;
+    launch_step(spl_topk_stretch_kernel, dim3(stretches, rows), dim3(256), 0, e->stream, (const float *)e->logits, e->logits_ld, vocab_limit, k, lists);
+    launch_step(spl_topk_merge_kernel, dim3(rows), dim3(32), staged ? staged_bytes : size_t(stretches), e->stream, (const float *)e->logits, e->logits_ld, (const uint2 *)lists,
+                stretches, k, staged ? 1 : 0, ids_dev, reinterpret_cast<float *>(ids_dev) + picks);
     const spl_status launched = check_launch(e, "top-k");
     if (launched != SPL_OK) return launched;
-    SPL_CUDA(cudaMemcpyAsync(e->topk_host, e->topk_picks, picks * 8, cudaMemcpyDeviceToHost, e->stream));
+    SPL_CUDA(cudaMemcpyAsync(e->topk_host, ids_dev, picks * 8, cudaMemcpyDeviceToHost, e->stream));
     SPL_CUDA(cudaStreamSynchronize(e->stream));
     std::memcpy(ids, e->topk_host, picks * 4);
     std::memcpy(values, e->topk_host + picks, picks * 4);

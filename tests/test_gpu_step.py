@@ -371,6 +371,25 @@ def test_topk_on_the_device_and_sampling_from_it(toks):
         engine.topk(65)
 
 
+def test_topk_takes_no_device_memory_of_its_own(toks):
+    """An engine laid out to fill the device has its scratch from the start: the first top-k of 2,048 rows at the largest k takes none (its lists
+    would be 4 MB here, 32 MB for the 27B vocabulary)."""
+    import torch
+    g = S.tiny_geometry()
+    model = O.Model(O.tiny_geometry())
+    small = S.Engine(g, S.EngineConfig(max_slots=1, max_rows=8, kv_pages=1, max_context=256))
+    small.load_model(model)
+    small.step([S.EngineRow(0, toks[0], 0, True)])
+    small.topk(64)                                   # loads the kernels' code
+    engine = S.Engine(g, S.EngineConfig(max_slots=1, max_rows=2048, kv_pages=9, max_context=2304, max_logit_rows=2048))
+    engine.load_model(model)
+    engine.step([S.EngineRow(0, toks[i % 500], i, True) for i in range(2048)])
+    before = torch.cuda.mem_get_info()[0]
+    ids, _ = engine.topk(64)
+    assert torch.cuda.mem_get_info()[0] == before
+    assert np.array_equal(ids[:, 0], engine.argmax())
+
+
 class _SparseHead:
     """The tiny model with a head whose rows are zero but for `kept`: every other logit is exactly zero."""
 
