@@ -78,13 +78,26 @@ __global__ void spl_repack_gguf_kernel(const unsigned char *__restrict__ native,
     }
 }
 
-// Stages of weight blocks in flight: as many as there are dequant sets (more, five at 16 rows, were measured: no change). The
-// sets take the half-stage units in turn, so a set works in two stages of every three: with three slots it comes back to the
-// same two, and has itself seen a slot's last phase when it waits for the next. With a ring of another length it would
-// meet slots whose last phase it skipped, and where that copy was still under way (the next slot's had overtaken it) the wait for
-// the coming phase would be answered by the one before: the set would read the old tenant and hand its slot back early
-// (at two stages, 64 rows of the byte-wide types: a wrong sum, or a launch failure in the blocks after it).
+// Stages of weight blocks in flight, and the dequant sets that read them. The sets take the half-stage units in turn, and a set's wait for a stage is
+// told from the wait before it only if the set has itself seen the slot's last phase: where it skipped that phase and its copy is still under
+// way (the next slot's has overtaken it), the wait is answered by the phase before, the set reads the old tenant and hands its slot
+// back early. With three sets and three slots a set comes back to the same two slots every six units. With two slots (64 rows of the byte-wide
+// types once had them) it met slots whose last phase it had skipped, and sums were wrong or a launch failed; five slots would skip phases too, so more
+// stages means six.
+#define SPL_GG_SETS 3
 #define SPL_GG_CSTAGES 3
+constexpr bool spl_gguf_ring_holds(int stages, int sets) {
+    for (int set = 0; set < sets; ++set) {
+        int seen[16] = {};                                    // phases of a slot this set has waited for
+        for (int un = set; un < 4 * stages * sets; un += sets) {
+            const int j = un / 2, slot = j % stages, phase = j / stages;
+            if (phase > seen[slot]) return false;
+            seen[slot] = phase + 1;
+        }
+    }
+    return true;
+}
+static_assert(SPL_GG_CSTAGES <= 16 && spl_gguf_ring_holds(SPL_GG_CSTAGES, SPL_GG_SETS), "a dequant set would skip a phase of a weight slot it comes back to");
 // The 128-row block (steps of more than 64 rows, where it saves waves of blocks) forms a weight once for twice the rows of the 64-row block. Its
 // activations come a unit (two groups, 32 KB) a stage, two units a stage for the others. Tensor memory: two accumulators of
 // 128 columns and the four operand slots of 64 fill the 512. A step with a 200-row Q4_K prompt of the 27B shape: 46.2 -> 33.7 ms (of it the SiLU
@@ -92,7 +105,7 @@ __global__ void spl_repack_gguf_kernel(const unsigned char *__restrict__ native,
 __host__ __device__ constexpr int spl_gguf_stage_units(int rn) { return rn >= 128 ? 1 : 2; }
 // Stages of activations: four, or three where the widened blocks beside 64 or 128 rows leave no room for a fourth.
 __host__ __device__ constexpr int spl_gguf_bstages(int rn, int format) { return (rn >= 64 && format != SPL_GGUF_Q4K) ? 3 : 4; }
-#define SPL_GG_THREADS 480       // warps 0-3, 8-11 and 4-7: three dequant sets; 12 copies; 13-14 tensor-core issue
+#define SPL_GG_THREADS 480       // warps 0-3, 8-11 and 4-7: the dequant sets; 12 copies; 13-14 tensor-core issue
 __host__ __device__ constexpr size_t spl_gguf_smem_bytes(int rn, int format) {
     return 1024 + size_t(SPL_GG_CSTAGES) * spl_gguf_pieces(format) * 2048 + size_t(spl_gguf_bstages(rn, format)) * spl_gguf_stage_units(rn) * 2 * rn * 128 + 1024;
 }
@@ -327,7 +340,7 @@ spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfl
     } else {
         const int quarter = warp & 3, col = quarter * 32 + lane, set = warp < 4 ? 0 : warp >= 8 ? 1 : 2;
         const uint32_t lane_base = uint32_t(quarter * 32) << 16;
-        for (int un = set; un < units && ok; un += 3) {
+        for (int un = set; un < units && ok; un += SPL_GG_SETS) {
             const int j = un >> 1, half = un & 1, sc = j % CST;
             ok = spl_mbar_wait(&full_c[sc], (j / CST) & 1);
             if (!ok) break;
@@ -359,7 +372,7 @@ spl_gemm_gguf_tc_kernel(const unsigned char *__restrict__ blocks, const __nv_bfl
             float *dst = is_split ? partials + size_t(split) * rows_padded * out_ld : out;
 #pragma unroll
             for (int cb = 0; cb < RN / 16; ++cb) {
-                if (cb % 3 != set) continue;
+                if (cb % SPL_GG_SETS != set) continue;
                 const int c0 = cb * 16;
                 float total[16];
 #pragma unroll

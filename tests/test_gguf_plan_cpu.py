@@ -2,6 +2,9 @@
 
 A weight is formed once a block, so blocks of 128 rows convert half of what blocks of 64 do, but each takes longer (about 1.25 to 1.5 times): they
 are right where they save more than that in waves of blocks, and never where they save no wave."""
+import os
+import re
+
 import pytest
 
 from splosh_b200.engine import EngineError, debug_gguf_plan
@@ -47,3 +50,23 @@ def test_bad_arguments_are_refused():
     for n, k, rows, sms in ((0, 256, 1, 148), (128, 0, 1, 148), (128, 100, 1, 148), (128, 256, 0, 148), (128, 256, 1, 0)):
         with pytest.raises(EngineError):
             debug_gguf_plan("Q4_K", n, k, rows, sms)
+
+
+def skips_a_phase(stages, sets):
+    """The weight ring's schedule: dequant set s takes the half-stage units s, s + sets, ... A set that comes to a slot for phase p
+    has to have waited for phase p - 1 itself, or never have been due there before: its barrier tells two phases apart, no more."""
+    for s in range(sets):
+        last = {}
+        for unit in range(s, 24 * stages * sets, sets):
+            slot, phase = unit // 2 % stages, unit // 2 // stages
+            if phase not in (last.get(slot, -1), last.get(slot, -1) + 1):
+                return True
+            last[slot] = phase
+    return False
+
+
+def test_no_dequant_set_skips_a_phase_of_the_weight_ring():
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "splosh_b200", "csrc", "spl_gemm_gguf.cuh")
+    define = dict(re.findall(r"#define (SPL_GG_SETS|SPL_GG_CSTAGES) (\d+)", open(path).read()))
+    assert not skips_a_phase(int(define["SPL_GG_CSTAGES"]), int(define["SPL_GG_SETS"]))
+    assert skips_a_phase(2, 3) and skips_a_phase(4, 3) and skips_a_phase(5, 3) and not skips_a_phase(6, 3)
