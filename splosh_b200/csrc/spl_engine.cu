@@ -75,6 +75,7 @@ struct spl_engine {
     size_t slot_floats = 0;
     bool gdn_out_file_order = false;      // spl_weights_gguf_file_order
     int gdn_chunk_min = SPL_GDN_CHUNK_MIN;      // ordinary runs at least this long take the chunked gated-delta scan (spl_debug_gdn_chunk_min)
+    int gguf_block_rows = 0;      // test switch (spl_debug_gguf_block_rows)
     int sms = 148;
     int rows_padded = 0, logit_rows_padded = 0;
     int *tc_error = nullptr;
@@ -402,7 +403,7 @@ bool launch_gemm_rows(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand 
 }
 
 // Where a cut GGUF GEMM's blocks leave their partial sums, the launch's error words, the device's SM count.
-struct GgufScratch { float *partials; size_t floats; int *error_flag; int sms; };
+struct GgufScratch { float *partials; size_t floats; int *error_flag; int sms; int block_rows = 0; };      // block_rows: a test's choice, 0 for the rule's
 
 // The pieces of a GGUF tensor's contraction for `rows` rows: the q4 rule in units of four groups, a piece a whole number of super-blocks. Blocks
 // of 64 and of 128 rows are cut alike, as suits blocks of 64, and both keep two accumulators: the order of a sum, and so the output to the
@@ -421,6 +422,7 @@ int gguf_pieces(const SplGgufDev &w, int rows, int rows_padded, const GgufScratc
 // 34,816 x 5,120 (8 waves or 4): 184 -> 121, 189 -> 140, 181 -> 143 us; at 129 rows (6 or 4): 141 -> 119, 145 -> 137, 139 -> 141 us.
 int gguf_operand_rn(int rows, std::initializer_list<const SplGgufDev *> readers, const GgufScratch &scratch) {
     if (rows <= 64) return operand_rn(rows);
+    if (scratch.block_rows) return scratch.block_rows;
     double cost[2] = {0, 0};
     for (const SplGgufDev *w : readers) {
         const double wide = w->format == SPL_GGUF_Q4K ? 1.25 : w->format == SPL_GGUF_Q5K ? 1.40 : 1.52;
@@ -539,7 +541,7 @@ spl_status enqueue_step(spl_engine *e, const spl_tables *t) {
     const int H = g.hidden;
     // GEMM operands of this step: row blocks of rn rows, in the tile layout the tensor cores read.
     // (The blocks of a model have two shapes: its first gated-delta block and its first attention block stand for them.)
-    const GgufScratch gscratch{e->partials, e->partial_floats, e->tc_error, e->sms};
+    const GgufScratch gscratch{e->partials, e->partial_floats, e->tc_error, e->sms, e->gguf_block_rows};
     const LayerWeights &first = e->layers[0], &fourth = e->layers[std::min<size_t>(3, e->layers.size() - 1)];
     const int rn = gguf ? gguf_operand_rn(R, {&first.g_in_proj, &fourth.g_in_proj, &first.g_gate_up}, gscratch) : operand_rn(R), blocks = (R + rn - 1) / rn;
     const int core_rn = gguf ? gguf_operand_rn(R, {&first.g_out_proj, &fourth.g_out_proj}, gscratch) : rn, core_blocks = (R + core_rn - 1) / core_rn;
@@ -1436,6 +1438,12 @@ spl_status spl_debug_gguf_plan(int32_t format, int32_t n, int32_t k, int32_t row
     const GgufScratch scratch{nullptr, SIZE_MAX, nullptr, sms};
     *block_rows = gguf_operand_rn(rows, {&w}, scratch);
     *pieces = gguf_pieces(w, rows, (rows + *block_rows - 1) / *block_rows * *block_rows, scratch);
+    return SPL_OK;
+}
+
+spl_status spl_debug_gguf_block_rows(spl_engine *e, int32_t rows) {
+    if (!e || (rows != 0 && rows != 64 && rows != 128)) return SPL_ERR_INVALID_ARGUMENT;
+    e->gguf_block_rows = rows;
     return SPL_OK;
 }
 

@@ -212,6 +212,7 @@ def lib():
             "spl_debug_kv_store": (i32, [vp, i32]),
             "spl_debug_gdn_chunk_min": (i32, [vp, i32]),
             "spl_debug_gguf_plan": (i32, [i32, i32, i32, i32, i32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
+            "spl_debug_gguf_block_rows": (i32, [vp, i32]),
             "spl_debug_pair_blocks": (i32, [vp, i32]),
             "spl_debug_wait_budget": (i32, [vp, C.c_int64]),
             "spl_debug_drop_weight_stage": (i32, [vp, i32]),
@@ -713,6 +714,10 @@ class Engine:
     def debug_gdn_chunk_min(self, rows):
         """Ordinary runs of at least `rows` rows (default 512) take the chunked gated-delta scan."""
         self._check(lib().spl_debug_gdn_chunk_min(self.handle, int(rows)))
+
+    def debug_gguf_block_rows(self, rows=0):
+        """GGUF GEMMs of steps of more than 64 rows in blocks of 64 or of 128 rows (0: by waves of blocks, the default)."""
+        self._check(lib().spl_debug_gguf_block_rows(self.handle, rows))
 
     def debug_pair_blocks(self, enabled=True):
         """Prompt chunks' GEMMs on the pair form of the 128-row block (default) or on the one-tile block."""

@@ -55,6 +55,42 @@ def test_gguf_weighted_step_matches_the_oracle(plain_norms, kinds):
     observed(f"GGUF-weighted step ({kinds[0]} blocks, {kinds[1]} embedding and head): max |logit - oracle| {worst:.3e} (<= {LOGIT_TOL})")
 
 
+@pytest.mark.parametrize("kinds", [("Q5_K", "Q6_K"), ("Q4_K", "Q6_K"), ("Q6_K", "Q4_K")])
+def test_steps_of_more_than_64_rows(plain_norms, kinds):
+    """Prompts of one and two blocks of 128 rows with ragged ends, a step with more than 64 logit rows, and one whose last block computes far fewer
+    rows than the operand holds (a decoder's rows in front of a prompt chunk without logits), over an inner dimension that leaves the SiLU kernel's last block
+    half empty: against the oracle, and in blocks of 64 and of 128 rows to the bit alike."""
+    g = S.Geometry(4, 256, 768, 2048, 8, 2, 128, 32, 2, 4, 128, 1e-6, 1e7)
+    cfg = S.EngineConfig(max_slots=3, max_rows=256, kv_pages=8, max_context=1024)
+    pair = Pair(g, cfg, gguf=kinds)
+    twins = []
+    for rows in (64, 128):
+        twin = S.Engine(g, cfg)
+        twin.load_gguf_model(pair.model)
+        twin.debug_gguf_block_rows(rows)
+        twins.append(twin)
+    toks = tokens_for(0xC0FFEE00, 800, g.vocab)
+    steps = [
+        [S.EngineRow(0, toks[i], i, i == 199) for i in range(200)],
+        [S.EngineRow(1, toks[200 + i], i, i % 2 == 1 or i > 60) for i in range(129)],
+        [S.EngineRow(0, toks[400 + i], 200 + i, True, True) for i in range(8)] + [S.EngineRow(2, toks[500 + i], i, False) for i in range(150)],
+        [S.EngineRow(2, toks[650 + i], 150 + i, i == 69) for i in range(70)],
+    ]
+    worst, live = 0.0, []
+    for rows in steps:
+        glogits, ologits = pair.step(rows)
+        live.append(int(pair.last_tables.live_rows))
+        worst = max(worst, np.abs(glogits - ologits).max())
+        assert np.abs(glogits - ologits).max() < LOGIT_TOL * max(1.0, np.abs(ologits).max())
+        for twin in twins:
+            twin.step(rows)
+            assert np.array_equal(twin.all_logits(), glogits)
+    assert live[2] == 8 and len(steps[2]) > 128       # one block of rows computed where the operand has two or three
+    with pytest.raises(S.EngineError):
+        twins[0].debug_gguf_block_rows(32)
+    observed(f"GGUF-weighted steps of 70 to 200 rows ({kinds[0]} blocks, {kinds[1]} embedding and head): max |logit - oracle| {worst:.3e} (<= {LOGIT_TOL})")
+
+
 def test_a_partly_converted_engine_refuses_to_step(plain_norms):
     g = geometry()
     cfg = S.EngineConfig(max_slots=1, max_rows=16, kv_pages=4, max_context=512)
