@@ -429,6 +429,58 @@ def test_topk_orders_equal_values_by_index_across_lanes_warps_and_stretches(toks
             assert list(ids[r]) == rid and np.array_equal(values[r], rvalues), (k, limit, r)
 
 
+def test_topk_of_nan_and_infinite_logits(toks):
+    """NaN and -inf are never picked, +inf is, in index order; rows with fewer than k of them keep the untouched slots (id 0 at -inf). A GGUF head
+    (fp16 products, no bias term) under a final norm whose weight overflows fp16 in one channel gives +inf, -inf and NaN by the sign of a
+    column's weight there."""
+    from helpers import to_oracle_geometry
+    from oracle import sampler as OS
+    g = S.Geometry(4, 256, 512, 20000, 8, 2, 128, 32, 2, 4, 128, 1e-6, 1e7)
+    model = O.Model(to_oracle_geometry(g)).to_gguf("Q4_K", "Q6_K")
+
+    class Overflowing:
+        def vec(self, layer, kind):
+            bits = model.vec(layer, kind)
+            if kind == "final_norm":
+                bits = bits.copy()
+                bits[7] = 0x7149                       # 1e30 in bf16
+            return bits
+
+        def __getattr__(self, name):
+            return getattr(model, name)
+
+    engine = S.Engine(g, S.EngineConfig(max_slots=1, max_rows=32, kv_pages=2, max_context=256))
+    engine.load_gguf_model(Overflowing())
+    engine.step([S.EngineRow(0, toks[i] % g.vocab, i, i >= 2) for i in range(5)])
+    logits = engine.all_logits()
+    assert np.isnan(logits).any() and (logits == np.inf).any() and (logits == -np.inf).any()
+    short = 0
+    for k, limit in ((64, g.vocab), (20, 8193), (40, 60), (64, 64), (1, 1), (3, 3), (30, 1030)):
+        ids, values = engine.topk(k, limit)
+        for r in range(logits.shape[0]):
+            rid, rvalues = OS.topk_select(logits[r], limit, k)
+            assert list(ids[r]) == rid and np.array_equal(values[r], rvalues), (k, limit, r)
+            short += rvalues[-1] == -np.inf
+    assert short > 0
+
+
+def test_topk_of_vocabularies_wider_than_a_warps_lists(toks):
+    """A row of 98 stretches: several lists a lane in the merge, and at k = 64 more list entries than its block's shared memory takes."""
+    from oracle import sampler as OS
+    from splosh_b200 import synthetic
+    g = S.Geometry(4, 256, 512, 800000, 8, 2, 128, 32, 2, 4, 128, 1e-6, 1e7)
+    engine = S.Engine(g, S.EngineConfig(max_slots=1, max_rows=16, kv_pages=1, max_context=256))
+    synthetic.load_vectors(engine, 5)
+    engine.synthesize_q4(5)
+    engine.step([S.EngineRow(0, toks[i], i, i >= 3) for i in range(5)])
+    logits = engine.all_logits()
+    for k, limit in ((64, g.vocab), (62, g.vocab), (20, 270000), (64, 262145), (1, g.vocab)):
+        ids, values = engine.topk(k, limit)
+        for r in range(logits.shape[0]):
+            rid, rvalues = OS.topk_select(logits[r], limit, k)
+            assert list(ids[r]) == rid and np.array_equal(values[r], rvalues), (k, limit, r)
+
+
 def test_a_slot_moves_to_another_engine_through_state_and_kv_snapshots(toks):
     """exportState / exportKV / importState / importSlot (Engine.swift:870-1042). A conversation of 300 tokens plus one
     accepted 6-row speculative block (so the export has journal entries to fold in) moves from slot 0 of engine A to
