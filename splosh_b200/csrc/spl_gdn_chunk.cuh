@@ -25,8 +25,10 @@
 #include "spl_gdn.cuh"
 
 #define SPL_GDN_CHUNK 64           // tokens per chunk
-#define SPL_GDN_CHUNK_MIN 512      // ordinary runs at least this long take the chunked path by default: below about five chunks the
-                                   // per-token kernel is the faster one (a chunk costs it 83 us; the three kernels here 150 us + 50 us a chunk)
+// Ordinary runs at least this long take the chunked path by default. It is the faster one from about 80 rows (less time a gated-delta block: 26 us at
+// 96 rows, 57 at 128, 88 at 200, 183 at 301, 327 at 511), but it adds in another order, and 64 blocks carry the difference on: a 301-row prompt's logits
+// move by 2.9e-2 of their norm. The line keeps shorter prompts on the order of sums they have always had.
+#define SPL_GDN_CHUNK_MIN 512
 #define SPL_GDN_SLICES 8           // slices of the value dimension in the scan (16 values each)
 #define SPL_GDN_SLICE (SPL_GDN_D / SPL_GDN_SLICES)
 #define SPL_GDN_LD (SPL_GDN_D + 4)   // floats between rows of D in shared memory

@@ -100,8 +100,9 @@ constexpr bool spl_gguf_ring_holds(int stages, int sets) {
 static_assert(SPL_GG_CSTAGES <= 16 && spl_gguf_ring_holds(SPL_GG_CSTAGES, SPL_GG_SETS), "a dequant set would skip a phase of a weight slot it comes back to");
 // The 128-row block (steps of more than 64 rows, where it saves waves of blocks) forms a weight once for twice the rows of the 64-row block. Its
 // activations come a unit (two groups, 32 KB) a stage, two units a stage for the others. Tensor memory: two accumulators of
-// 128 columns and the four operand slots of 64 fill the 512. A step with a 200-row Q4_K prompt of the 27B shape: 46.2 -> 33.7 ms (of it the SiLU
-// kernel's larger blocks and the top-k).
+// 128 columns and the four operand slots of 64 fill the 512. A step with a 200-row Q4_K prompt of the 27B shape: 44.8 -> 35.9 ms
+// (37.0 with the cut that suits blocks of 64 kept). At 200 rows L2 delivers 6.8 TB/s, most of it activations, to 34,816 x 5,120's blocks, with the tensor
+// pipe 41 % and the conversion's 46 % busy.
 __host__ __device__ constexpr int spl_gguf_stage_units(int rn) { return rn >= 128 ? 1 : 2; }
 // Stages of activations: four, or three where the widened blocks beside 64 or 128 rows leave no room for a fourth.
 __host__ __device__ constexpr int spl_gguf_bstages(int rn, int format) { return (rn >= 64 && format != SPL_GGUF_Q4K) ? 3 : 4; }
@@ -447,7 +448,7 @@ __global__ void spl_embed_gguf_kernel(const unsigned char *__restrict__ table, i
 
 // act = bf16(silu(gate) * up) of an unfused gate|up output [rows][2 inter] (gate columns first) as the down projection's
 // operand with its per-64 sums (Sources/Shaders/engine.metal:200-219). Grid (groups of 64 in eights, rows), 256 threads: a warp a group (a block of
-// one warp each is 54,400 blocks for a 200-row prompt of the 27B shape, and what that costs is their launch).
+// one warp each is 54,400 blocks for a 200-row prompt of the 27B shape, and what that costs is their launch: its step 37.0 -> 33.8 ms).
 __global__ void __launch_bounds__(256) spl_swiglu_kernel(const float *__restrict__ gate_up, int ld, int inter, SplOperand out) {
     spl_grid_begin();
     const int group = blockIdx.x * 8 + (threadIdx.x >> 5), row = blockIdx.y, lane = threadIdx.x & 31, n = group * 64 + 2 * lane;
