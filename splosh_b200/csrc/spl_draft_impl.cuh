@@ -137,7 +137,7 @@ static spl_status draft_linear(spl_draft *d, const uint16_t *bf16, int rows, int
     spl_status s = alloc_q4(e, t->q, rows, inner);
     if (s == SPL_OK) s = upload_q4_into(e, t->q, 0, rows, inner, packed.data(), scales.data(), biases.data(), false);
     size_t need = 0;
-    for (int rn : {16, 32, 64, 128}) need = std::max(need, gemm_slot_floats(t->q, e->sms, rn, std::max(1, e->c.max_rows / 128), false, false));
+    need = std::max(need, gemm_slot_floats(t->q, e->sms, 128, std::max(1, e->c.max_rows / 128), false, false));
     if (s == SPL_OK && need > e->slot_floats) {
         cudaFree(e->slots); e->slots = nullptr;
         if (cudaMalloc(reinterpret_cast<void **>(&e->slots), need * 4) != cudaSuccess) s = e->fail(SPL_ERR_ALLOCATION_FAILED, "GEMM scratch");

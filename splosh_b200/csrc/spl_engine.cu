@@ -18,6 +18,7 @@
 #include "spl_gdn.cuh"
 #include "spl_gdn_chunk.cuh"
 #include "spl_gemm_tc.cuh"
+#include "spl_gemm_narrow.cuh"
 #include "spl_host.h"
 
 namespace {
@@ -230,11 +231,13 @@ struct GemmScratch { float *slots; size_t slot_floats; int *error_flag; int sms;
 
 // The kernels that need more than the default shared memory, opted in on the current device (the attribute is per device).
 template <int RN> void configure_gemm() {
-    cudaFuncSetAttribute(spl_gemm_q4_tc_kernel<RN, SPL_TC_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_smem_bytes(RN)));
-    cudaFuncSetAttribute(spl_gemm_q4_tc_kernel<RN, SPL_TC_EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_smem_bytes(RN)));
-    cudaFuncSetAttribute(spl_gemm_q4_tc_kernel<RN, SPL_TC_FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_smem_bytes(RN)));
-    if constexpr (RN < 128) cudaFuncSetAttribute(spl_gemm_q4_narrow_kernel<RN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_smem_bytes(RN)));
-    if constexpr (RN == 128) cudaFuncSetAttribute(spl_gemm_q4_narrow_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_pair_smem_bytes()));
+    if constexpr (RN == 128) {
+        cudaFuncSetAttribute(spl_gemm_q4_tc_kernel<RN, SPL_TC_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_smem_bytes(RN)));
+        cudaFuncSetAttribute(spl_gemm_q4_tc_kernel<RN, SPL_TC_EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_smem_bytes(RN)));
+        cudaFuncSetAttribute(spl_gemm_q4_tc_kernel<RN, SPL_TC_FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_smem_bytes(RN)));
+    }
+    if constexpr (RN < 128) cudaFuncSetAttribute(spl_gemm_q4_narrow_kernel<RN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_narrow_smem_bytes(RN)));
+    if constexpr (RN == 128) cudaFuncSetAttribute(spl_gemm_q4_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_tc_pair_smem_bytes()));
 }
 template <int RN, int FMT> void configure_gguf() { cudaFuncSetAttribute(spl_gemm_gguf_tc_kernel<RN, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_gguf_smem_bytes(RN, FMT))); }
 template <int HD, int PER_KV> void configure_scan() { cudaFuncSetAttribute(spl_attn_scan_kernel<HD, PER_KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_attn_smem_bytes(HD, spl_attn_nq(PER_KV)))); }
@@ -275,7 +278,7 @@ struct GemmCut { int pieces, splits; };
 GemmCut gemm_cut(const SplQ4Dev &w, int sms, int rn, int row_blocks, bool whole) {
     const int stages = w.k / (64 * spl_tc_super(rn));
     int best = 1; double best_cost = 1e30;
-    for (int s = 1; s <= stages && s <= 16 && !(whole && s > 1); ++s) {
+    for (int s = 1; s <= stages && s <= (rn < 128 ? SPL_NARROW_CLUSTER : 16) && !(whole && s > 1); ++s) {
         const int per = (stages + s - 1) / s;
         if (s > 1 && per < 2) break;
         const int waves = (w.tiles * s * row_blocks + sms - 1) / sms;
@@ -303,18 +306,15 @@ int pair_splits(const SplQ4Dev &w, int sms, int row_blocks, bool whole) {
     return (stages + per - 1) / per;
 }
 
-// Floats of scratch a GEMM on `w` may leave for its second kernel: the wide block's slots, or the narrow block's
+// Floats of scratch a GEMM on `w` may leave for its second kernel: the one-tile 128-row block's slots, or the pair form's
 // partials[split][row][column] (cut tiles, and every tile when the output feeds a deferred norm: `emit`).
 size_t gemm_slot_floats(const SplQ4Dev &w, int sms, int rn, int row_blocks, bool emit, bool whole) {
+    if (rn < 128) return 0;          // the blocks of the narrow kernel's cut tiles meet in a cluster
     const GemmCut cut = gemm_cut(w, sms, rn, row_blocks, whole);
-    if (rn >= 128) {
-        // The pair form leaves cut contractions, and an output that feeds a deferred norm, to the second kernel.
-        const int ps = pair_splits(w, sms, row_blocks, whole);
-        const size_t pair = (ps > 1 || (ps == 1 && emit)) ? size_t(ps) * row_blocks * rn * w.ld : 0;
-        return std::max(spl_tc_slot_floats(cut.pieces, cut.splits, row_blocks, rn), pair);
-    }
-    const int stages = w.k / 256, per = (stages + cut.splits - 1) / cut.splits, splits = (stages + per - 1) / per;
-    return (splits > 1 || emit) ? size_t(splits) * row_blocks * rn * w.ld : 0;
+    // The pair form leaves cut contractions, and an output that feeds a deferred norm, to the second kernel.
+    const int ps = pair_splits(w, sms, row_blocks, whole);
+    const size_t pair = (ps > 1 || (ps == 1 && emit)) ? size_t(ps) * row_blocks * rn * w.ld : 0;
+    return std::max(spl_tc_slot_floats(cut.pieces, cut.splits, row_blocks, rn), pair);
 }
 
 template <int RN>
@@ -336,23 +336,25 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
     a.emit_weight = x.emit_weight; a.emit_out = emit_out; a.emit_squares = x.emit_squares;
     const dim3 grid(cut.pieces * row_blocks), block(SPL_TC_THREADS);
     if constexpr (RN < 128) {
-        // The narrow block: a tile's contraction in `splits` runs of whole stages. A cut GEMM, and one whose output feeds a
-        // deferred norm, leave partial sums for the second kernel.
+        // The narrow block: a cut tile's pieces are a cluster of blocks, one tile a cluster; a block of an uncut tensor stays and takes every gridDim.x-th tile.
         const int stages = w.k / 256, per = (stages + cut.splits - 1) / cut.splits, splits = (stages + per - 1) / per;
-        const bool second = splits > 1 || x.emit_weight != nullptr;
-        const size_t rows_padded = size_t(op.blocks) * RN;
-        if (second && size_t(splits) * rows_padded * w.ld > scratch.slot_floats) return false;
-        launch_step(spl_gemm_q4_narrow_kernel<RN>, dim3(w.tiles, splits, row_blocks), block, spl_tc_smem_bytes(RN), stream, (const uint32_t *)w.codes, (const uint32_t *)w.sb, op.values, op.sums,
-                    out, w.ld, second ? (const float *)nullptr : residual, second ? scratch.slots : (float *)nullptr, rows, op.blocks, w.k / 64, per * 4, scratch.error_flag, w.interleave,
-                    a.act_out, a.fuse, x.in_squares, x.in_dim / 64, float(x.in_dim), x.eps, g_drop_weight_stage);
+        SplNarrowArgs n = {};
+        n.codes = reinterpret_cast<const unsigned char *>(w.codes); n.sb = reinterpret_cast<const unsigned char *>(w.sb);
+        n.act = reinterpret_cast<const unsigned char *>(op.values); n.means = reinterpret_cast<const unsigned char *>(op.sums);
+        n.out = out; n.residual = residual; n.out_ld = w.ld; n.rows = rows; n.groups = w.k / 64; n.tiles = w.tiles; n.splits = splits;
+        n.interleave = w.interleave; n.fuse = a.fuse; n.drop = g_drop_weight_stage; n.error_flag = scratch.error_flag;
+        n.in_squares = x.in_squares; n.in_groups = x.in_dim / 64; n.in_dim = float(x.in_dim); n.eps = x.eps;
+        n.act_out = a.act_out; n.emit_weight = x.emit_weight; n.emit_out = emit_out; n.emit_squares = x.emit_squares;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(splits > 1 ? w.tiles * splits : std::min(w.tiles, scratch.sms)); cfg.blockDim = dim3(SPL_NARROW_THREADS); cfg.dynamicSmemBytes = spl_narrow_smem_bytes(RN); cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = splits; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 2;
+        cudaLaunchKernelEx(&cfg, spl_gemm_q4_narrow_kernel<RN>, n);
         if (launches) ++*launches;
-        if (second) {
-            if (scratch.timed) { profile_end(scratch.timed); profile_begin(scratch.timed, KLASS_ELEMENTWISE, 0); }
-            else if (launches) ++*launches;
-            const long long warps = (long long)rows * ((w.ld + 63) / 64);
-            launch_step(spl_gemm_fixup_rows_kernel, dim3(int(std::min<long long>((warps + 7) / 8, 8LL * scratch.sms))), dim3(256), 0, stream, (const float *)scratch.slots, splits, int(rows_padded), rows, w.ld,
-                        residual, out, x.emit_weight, emit_out, x.emit_squares);
-        }
         return true;
     }
     if constexpr (RN == 128) {
@@ -363,7 +365,7 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
             const bool second = splits > 1 || x.emit_weight != nullptr;
             const size_t rows_padded = size_t(op.blocks) * RN;
             if (second && size_t(splits) * rows_padded * w.ld > scratch.slot_floats) return false;
-            launch_step(spl_gemm_q4_narrow_kernel<128, true>, dim3(((w.tiles + 1) / 2) * row_blocks, splits), block, spl_tc_pair_smem_bytes(), stream, (const uint32_t *)w.codes, (const uint32_t *)w.sb, op.values, op.sums,
+            launch_step(spl_gemm_q4_pair_kernel, dim3(((w.tiles + 1) / 2) * row_blocks, splits), block, spl_tc_pair_smem_bytes(), stream, (const uint32_t *)w.codes, (const uint32_t *)w.sb, op.values, op.sums,
                         out, w.ld, second ? (const float *)nullptr : residual, second ? scratch.slots : (float *)nullptr, rows, op.blocks, w.k / 64, per * 4, scratch.error_flag, w.interleave,
                         a.act_out, a.fuse, x.in_squares, x.in_dim / 64, float(x.in_dim), x.eps, g_drop_weight_stage);
             if (launches) ++*launches;
@@ -377,18 +379,20 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
             return true;
         }
     }
-    if (x.fuse_act) launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_FUSE>, grid, block, spl_tc_smem_bytes(RN), stream, a);
-    else if (x.emit_weight && cut.splits == 1) launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_EMIT>, grid, block, spl_tc_smem_bytes(RN), stream, a);
-    else launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_PLAIN>, grid, block, spl_tc_smem_bytes(RN), stream, a);
-    if (launches) ++*launches;
-    if (cut.splits > 1) {
-        // The second kernel of a cut GEMM: the slots' sum in the order of the contraction, the residual, the output, the emitted operand.
-        if (scratch.timed) { profile_end(scratch.timed); profile_begin(scratch.timed, KLASS_ELEMENTWISE, 0); }
-        else if (launches) ++*launches;
-        const long long warps = (long long)rows * w.tiles * 2;
-        const int blocks = int(std::min<long long>((warps + 7) / 8, 8LL * scratch.sms));
-        launch_step(spl_gemm_fixup_kernel, dim3(blocks), dim3(256), 0, stream, (const float *)scratch.slots, cut.splits, cut.pieces, RN, rows, w.tiles, w.ld, w.interleave,
-                    residual, out, x.emit_weight, emit_out, x.emit_squares);
+    if constexpr (RN == 128) {
+        if (x.fuse_act) launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_FUSE>, grid, block, spl_tc_smem_bytes(RN), stream, a);
+        else if (x.emit_weight && cut.splits == 1) launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_EMIT>, grid, block, spl_tc_smem_bytes(RN), stream, a);
+        else launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_PLAIN>, grid, block, spl_tc_smem_bytes(RN), stream, a);
+        if (launches) ++*launches;
+        if (cut.splits > 1) {
+            // The second kernel of a cut GEMM: the slots' sum in the order of the contraction, the residual, the output, the emitted operand.
+            if (scratch.timed) { profile_end(scratch.timed); profile_begin(scratch.timed, KLASS_ELEMENTWISE, 0); }
+            else if (launches) ++*launches;
+            const long long warps = (long long)rows * w.tiles * 2;
+            const int blocks = int(std::min<long long>((warps + 7) / 8, 8LL * scratch.sms));
+            launch_step(spl_gemm_fixup_kernel, dim3(blocks), dim3(256), 0, stream, (const float *)scratch.slots, cut.splits, cut.pieces, RN, rows, w.tiles, w.ld, w.interleave,
+                        residual, out, x.emit_weight, emit_out, x.emit_squares);
+        }
     }
     return true;
 }
@@ -906,9 +910,7 @@ spl_status create(const spl_geometry *gp, const spl_config *cp, spl_engine *e) {
         std::vector<Use> all{{&e->head, false, false}};
         for (const LayerWeights &L : e->layers) { all.push_back({&L.in_proj, false, false}); all.push_back({&L.out_proj, true, false}); all.push_back({&L.gate_up, false, true}); all.push_back({&L.down, true, false}); }
         for (const Use &u : all)
-            for (int rn : {16, 32, 64, 128})
-                for (int rbs = 1; rbs <= (rn == 128 ? row_blocks : 1); ++rbs)
-                    e->slot_floats = std::max(e->slot_floats, gemm_slot_floats(*u.w, e->sms, rn, rbs, u.emit, u.whole));
+            for (int rbs = 1; rbs <= row_blocks; ++rbs) e->slot_floats = std::max(e->slot_floats, gemm_slot_floats(*u.w, e->sms, 128, rbs, u.emit, u.whole));
     }
     if ((s = device_alloc(e, &e->slots, e->slot_floats, &e->scratch_bytes)) != SPL_OK) return s;
     if (R >= SPL_GDN_CHUNK && !e->state.empty()) {
@@ -1972,8 +1974,7 @@ spl_status spl_tensor_create_q4(spl_engine *e, int32_t rows, int32_t inner, cons
     // The GEMM's scratch for partial sums has to hold this tensor's at any row count.
     size_t need = 0;
     const int row_blocks = std::max(1, e->c.max_rows / 128);
-    for (int rn : {16, 32, 64, 128})
-        for (int rbs = 1; rbs <= (rn == 128 ? row_blocks : 1); ++rbs) need = std::max(need, gemm_slot_floats(t->q, e->sms, rn, rbs, false, false));
+    for (int rbs = 1; rbs <= row_blocks; ++rbs) need = std::max(need, gemm_slot_floats(t->q, e->sms, 128, rbs, false, false));
     if (s == SPL_OK && need > e->slot_floats) {
         cudaFree(e->slots); e->slots = nullptr;
         if (cudaMalloc(reinterpret_cast<void **>(&e->slots), need * 4) != cudaSuccess) s = e->fail(SPL_ERR_ALLOCATION_FAILED, "GEMM scratch");

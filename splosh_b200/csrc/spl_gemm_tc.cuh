@@ -32,8 +32,9 @@
 //
 // Device layout of a weight (private to this library): for each tile of 128 output columns and each
 // group, 4,096 bytes of codes [half h][column n][16 bytes] holding k = 64 g + 32 h + 0..31, each
-// 32-bit word's nibbles in the order [k0 k2 k4 k6 k1 k3 k5 k7] so that (word >> 4j) & 0x000F000F is
-// the pair of codes (k_2j, k_2j+1); and 128 words (scale | bias << 16) per (tile, group).
+// 32-bit word's nibbles in the order [k0 k2 k4 k7 k1 k3 k5 k6] and the word rotated left by six, so that the pairs (k0, k1), (k2, k3), (k4, k5), (k6, k7)
+// come to mantissa bits 6-9 of its two halves by no shift, one of 4 to the right, a rotation by a byte and a shift of 4 to the left;
+// and 128 words (scale | bias << 16) per (tile, group).
 #pragma once
 #include "spl_common.cuh"
 
@@ -83,6 +84,10 @@ struct SplOperand {
         const __half2 pair = __halves2half2(hi, lo);
         const uint32_t bits = *reinterpret_cast<const uint32_t *>(&pair);
         const int rb = row >> (31 - __clz(rn)), r = row & (rn - 1), kk = 4 * (g & 15);
+        if (rn < 128) {        // blocks of up to 64 rows: sixteen bytes a row and pair of groups (spl_gemm_narrow.cuh)
+            *reinterpret_cast<uint2 *>(reinterpret_cast<unsigned char *>(sums) + ((size_t(g >> 1) * blocks + rb) * rn + r) * 16 + (g & 1) * 8) = make_uint2(bits, bits);
+            return;
+        }
         __half *tile = reinterpret_cast<__half *>(sums) + (size_t(g >> 4) * blocks + rb) * (size_t(rn) * 64);
         *reinterpret_cast<uint2 *>(tile + size_t(r >> 3) * 512 + (r & 7) * 64 + (((kk >> 3) ^ (r & 7)) << 3) + (kk & 7)) = make_uint2(bits, bits);
     }
@@ -96,13 +101,14 @@ __global__ void spl_repack_q4_kernel(const uint32_t *__restrict__ packed, const 
     for (size_t idx = blockIdx.x * size_t(blockDim.x) + threadIdx.x; idx < total; idx += size_t(gridDim.x) * blockDim.x) {
         const int row = int(idx / words), w = int(idx % words);
         const uint32_t src = packed[idx];
-        // nibbles [0 1 2 3 4 5 6 7] -> [0 2 4 6 1 3 5 7]
+        // nibbles [0 1 2 3 4 5 6 7] -> [0 2 4 7 1 3 5 6], then a rotation by six bits
         uint32_t dst = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            dst |= ((src >> (8 * j)) & 0xFu) << (4 * j);
-            dst |= ((src >> (8 * j + 4)) & 0xFu) << (4 * j + 16);
+            dst |= ((src >> (8 * j)) & 0xFu) << (j < 3 ? 4 * j : 4 * j + 16);
+            dst |= ((src >> (8 * j + 4)) & 0xFu) << (j < 3 ? 4 * j + 16 : 4 * j);
         }
+        dst = (dst << 6) | (dst >> 26);
         int n = n0 + row;
         if (interleave > 0) { const int c = n < interleave ? n : n - interleave; n = (c >> 6) * 128 + ((c & 63) >> 4) * 32 + (n < interleave ? 0 : 16) + (c & 15); }
         const int tile = n >> 7, col = n & 127, g = w >> 3, h = (w >> 2) & 1, j = w & 3;
@@ -322,17 +328,14 @@ __device__ __forceinline__ void spl_set_barrier(int set) {
 #define SPL_TC_PAIR_CSTAGES 4
 #define SPL_TC_PAIR_AUNITS 3
 
-// The shape of a block by its row count RN (the N of its tcgen05.mma). Narrow blocks (16, 32, 64 rows: decode and verify
-// steps) take stages of four groups and two issuing warps with an accumulator each. The wide block (128 rows: prefill
-// chunks, one instruction is 128 x 128 x 16) takes stages of two groups, so that four stages of activations still fit
-// in shared memory, and one issuing warp with one accumulator: an instruction then keeps the tensor pipe 64 cycles and
-// one warp issues at that rate.
-__host__ __device__ constexpr int spl_tc_super(int rn) { return rn >= 128 ? 2 : 4; }          // groups per stage
-__host__ __device__ constexpr int spl_tc_issuers(int rn) { return rn >= 128 ? 1 : 2; }        // issuing warps = units per stage
+// The one-tile block of 128 rows (an instruction is 128 x 128 x 16): stages of two groups, so that four stages of activations still fit in shared
+// memory, and one issuing warp with one accumulator: an instruction then keeps the tensor pipe 64 cycles and one warp issues at that rate.
+__host__ __device__ constexpr int spl_tc_super(int rn) { return rn >= 128 ? 2 : 4; }          // groups per stage (four: the narrow block, spl_gemm_narrow.cuh)
+__host__ __device__ constexpr int spl_tc_issuers(int) { return 1; }        // issuing warps = units per stage
 // Stages of activations: held until the tensor core has finished with them. Stages of codes with their scale/bias
 // words: handed back as soon as they are in registers.
-__host__ __device__ constexpr int spl_tc_bstages(int rn) { return rn >= 64 ? 4 : 6; }
-__host__ __device__ constexpr int spl_tc_cstages(int rn) { return rn >= 64 ? 4 : 6; }
+__host__ __device__ constexpr int spl_tc_bstages(int) { return 4; }
+__host__ __device__ constexpr int spl_tc_cstages(int) { return 4; }
 __host__ __device__ constexpr size_t spl_tc_bstage_bytes(int rn) { return size_t(spl_tc_super(rn)) * size_t(rn) * 128; }
 #define SPL_TC_CONTROL_BYTES 4096       // barriers, row factors, the output stage's exchange cells
 __host__ __device__ constexpr size_t spl_tc_smem_bytes(int rn) {
@@ -789,13 +792,13 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {
                     const uint4 src = part == 0 ? lo[v] : hi[v];
-                    const uint32_t w4[4] = {src.x, src.y, src.z, src.w};
+                        const uint32_t w4[4] = {src.x, src.y, src.z, src.w};
                     uint32_t regs[16];
 #pragma unroll
                     for (int w = 0; w < 4; ++w)
                         asm volatile("{\n .reg .b32 xa, xb, xc, xd;\n"      // volatile: converted sixteen registers at a time, in step with the stores, not all up front
-                            " shl.b32 xa, %4, 6;\n shl.b32 xb, %4, 2;\n shr.b32 xc, %4, 2;\n shr.b32 xd, %4, 6;\n"
-                            " lop3.b32 xa, xa, 0x03C003C0, 0x4C004C00, 0xEA;\n"
+                            " shr.b32 xb, %4, 4;\n prmt.b32 xc, %4, 0, 0x0321;\n shl.b32 xd, %4, 4;\n"
+                            " lop3.b32 xa, %4, 0x03C003C0, 0x4C004C00, 0xEA;\n"
                             " lop3.b32 xb, xb, 0x03C003C0, 0x4C004C00, 0xEA;\n"
                             " lop3.b32 xc, xc, 0x03C003C0, 0x4C004C00, 0xEA;\n"
                             " lop3.b32 xd, xd, 0x03C003C0, 0x4C004C00, 0xEA;\n"
@@ -850,21 +853,18 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
     }
 }
 
-// ---- the narrow block (16, 32, 64 rows: decode and verify steps) -------------------------------
-// Grid (tiles, splits, row blocks), one tile's share of the contraction a block: groups [split x groups_per_split, ...)
-// (a multiple of four). With one split the block writes the output (or, `fuse`, the SiLU-gated operand of the next
-// GEMM); with more it leaves its partial sums in partials[split][row][column] for spl_gemm_fixup_rows_kernel. Its
-// output stage is stores only: a block reaches it while the others still stream weights at the memory's full rate,
-// and a load issued then waits behind megabytes of queued copies.
-template <int RN, bool PAIR = false>
+// ---- the pair form of the 128-row block: steps of more than 64 rows ---------------------------
+// Grid (pairs of tiles x row blocks, splits): two tiles of the weight a block, one share of the contraction (whole stages of two groups). With one split
+// the block writes the output (or, `fuse`, the SiLU-gated operand of the next GEMM); with more it leaves its partial sums in
+// partials[split][row][column] for spl_gemm_fixup_rows_kernel. Its output stage is stores only: a block reaches it while the others still stream
+// weights at the memory's full rate, and a load issued then waits behind megabytes of queued copies.
 __global__ void __launch_bounds__(SPL_TC_THREADS, 1)
-spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__restrict__ sb, const __nv_bfloat16 *__restrict__ act,
+spl_gemm_q4_pair_kernel(const uint32_t *__restrict__ codes, const uint32_t *__restrict__ sb, const __nv_bfloat16 *__restrict__ act,
                       const float *__restrict__ act_sums, float *out, int out_ld, const float *residual, float *partials,
                       int rows, int op_blocks, int groups, int groups_per_split, int *error_flag, int interleave, SplOperand act_out, int fuse,
                       const float *__restrict__ in_squares, int in_groups, float in_dim, float eps, int drop) {
-    static_assert(!PAIR || RN == 128, "the pair form is the 128-row block");
-    constexpr int GPS = PAIR ? 2 : SPL_TC_SUPER;       // groups of the contraction a stage covers (the pair form: two, for each of its two tiles)
-    constexpr int BST = PAIR ? SPL_TC_PAIR_BSTAGES : spl_tc_bstages(RN), CST = PAIR ? SPL_TC_PAIR_CSTAGES : spl_tc_cstages(RN), AUN = PAIR ? SPL_TC_PAIR_AUNITS : SPL_TC_AUNITS;
+    constexpr int RN = 128, GPS = 2;       // rows; groups of the contraction a stage covers, for each of the two tiles
+    constexpr int BST = SPL_TC_PAIR_BSTAGES, CST = SPL_TC_PAIR_CSTAGES, AUN = SPL_TC_PAIR_AUNITS;
     constexpr int BTILE = GPS * RN * 128, WSTAGE = SPL_TC_SUPER * 4096, QSTAGE = SPL_TC_SUPER * 128, TTILE = RN * 128;
     extern __shared__ unsigned char spl_tc_smem_raw[];
     // The swizzled activation tiles must sit on 1,024-byte boundaries.
@@ -885,17 +885,17 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
     constexpr int W_COPY = SPL_TC_SETS * 4, W_MMA0 = W_COPY + 1, W_COPYB = W_COPY + 2, W_MMA1 = W_COPY + 3;
     // The pair form's grid has pair and row block in one dimension, the row block the fast index (the splits in the second): the blocks that run together are then the row
     // blocks of a few pairs, and a pair's weights come from HBM once and from L2 for the other row blocks.
-    const int run_blocks = PAIR ? (rows + RN - 1) / RN : 1;
-    const int tile = PAIR ? int(blockIdx.x) / run_blocks : int(blockIdx.x), split = int(blockIdx.y), rb = PAIR ? int(blockIdx.x) % run_blocks : int(blockIdx.z);
+    const int run_blocks = (rows + RN - 1) / RN;
+    const int tile = int(blockIdx.x) / run_blocks, split = int(blockIdx.y), rb = int(blockIdx.x) % run_blocks;
     const int row_blocks = op_blocks;   // the operand's row blocks (>= the grid's)
     const int tiles_all = (out_ld + 127) / 128;
-    const int tile0 = PAIR ? 2 * tile : tile, tile1 = PAIR ? min(2 * tile + 1, tiles_all - 1) : tile;      // an odd tensor's last pair does its one tile twice
-    const bool has1 = !PAIR || 2 * tile + 1 < tiles_all;
+    const int tile0 = 2 * tile, tile1 = min(2 * tile + 1, tiles_all - 1);      // an odd tensor's last pair does its one tile twice
+    const bool has1 = 2 * tile + 1 < tiles_all;
     const int rows_padded = op_blocks * RN;
     const int g_first = split * groups_per_split;
     const int g_count = min(groups_per_split, groups - g_first);
     const int supers = (g_count + GPS - 1) / GPS;
-    const int units = PAIR ? 2 * supers : (g_count + 1) / 2;            // a unit = two groups of one tile = one hand-over from a dequant set
+    const int units = 2 * supers;            // a unit = two groups of one tile = one hand-over from a dequant set
     // Every block of a GEMM reads the same activation lines. Blocks therefore walk the contraction from
     // different starting points (the order of a sum of groups does not matter beyond fp32 rounding, and it
     // is a fixed function of the tile), so that at any moment they ask L2 for different lines.
@@ -908,19 +908,12 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
     // Stage j of the block's share of the contraction into slot sc of the code ring: its codes and scale/bias words. The pair
     // form brings two groups of each of its two tiles (tile 0's at the slot's start, tile 1's after them).
     auto copy_codes = [&](int sc, int j, int n) {
-        if (PAIR) {
-            spl_mbar_expect_tx(&full_c[sc], 2u * uint32_t(n) * (4096 + 512));
+        spl_mbar_expect_tx(&full_c[sc], 2u * uint32_t(n) * (4096 + 512));
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const size_t first = size_t(m ? tile1 : tile0) * groups + g_first + size_t(j) * GPS;
-                spl_bulk_g2s(w_ring + size_t(sc) * WSTAGE + m * (GPS * 4096), reinterpret_cast<const unsigned char *>(codes) + first * 4096, uint32_t(n) * 4096, &full_c[sc]);
-                spl_bulk_g2s(q_ring + sc * QSTAGE + m * (GPS * 128), sb + first * 128, uint32_t(n) * 512, &full_c[sc]);
-            }
-        } else {
-            const size_t first = size_t(tile) * groups + g_first + size_t(j) * GPS;
-            spl_mbar_expect_tx(&full_c[sc], uint32_t(n) * (4096 + 512));
-            spl_bulk_g2s(w_ring + size_t(sc) * WSTAGE, reinterpret_cast<const unsigned char *>(codes) + first * 4096, uint32_t(n) * 4096, &full_c[sc]);
-            spl_bulk_g2s(q_ring + sc * QSTAGE, sb + first * 128, uint32_t(n) * 512, &full_c[sc]);
+        for (int m = 0; m < 2; ++m) {
+            const size_t first = size_t(m ? tile1 : tile0) * groups + g_first + size_t(j) * GPS;
+            spl_bulk_g2s(w_ring + size_t(sc) * WSTAGE + m * (GPS * 4096), reinterpret_cast<const unsigned char *>(codes) + first * 4096, uint32_t(n) * 4096, &full_c[sc]);
+            spl_bulk_g2s(q_ring + sc * QSTAGE + m * (GPS * 128), sb + first * 128, uint32_t(n) * 512, &full_c[sc]);
         }
     };
     if (warp == W_COPY && lane == 0) {
@@ -961,7 +954,7 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
     const uint32_t tmem = *tmem_slot;                 // lane 0, first allocated column
     // Two accumulators, one per issuing warp (instructions of different warps are not ordered against each other);
     // the A ring, 64 columns a unit; the second-term operand, 8 columns a unit.
-    const uint32_t tmem_d = tmem, tmem_a = tmem + (PAIR ? 2 * RN : 128), tmem_aq = tmem_a + AUN * 64;
+    const uint32_t tmem_d = tmem, tmem_a = tmem + 2 * RN, tmem_aq = tmem_a + AUN * 64;
     bool ok = true;
 
     if (!(warp == W_COPY && lane == 0)) spl_grid_begin();     // the thread that copies weights first asks for some (below)
@@ -1036,8 +1029,8 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
         int slot = m, fa = m;                              // un % AUN, un % (2 AUN)
         uint32_t a_parity = 0;                             // (un / (2 AUN)) & 1
         for (int un = m; un < units && ok; un += 2) {
-            const int j0 = un >> 1, sbq = j0 % BST, n = min(GPS, g_count - j0 * GPS) - (PAIR ? 0 : 2 * m);     // groups of this unit: 1 or 2
-            const uint64_t b_desc = b_desc0 + uint64_t((sbq * BTILE + (PAIR ? 0 : m * 2 * RN * 128)) >> 4);      // the pair's two tiles meet the same activations
+            const int j0 = un >> 1, sbq = j0 % BST, n = min(GPS, g_count - j0 * GPS);     // groups of this unit: 1 or 2
+            const uint64_t b_desc = b_desc0 + uint64_t((sbq * BTILE) >> 4);      // the pair's two tiles meet the same activations
             const uint32_t a_base = tmem_a + slot * 64;
             // The stage's share of the second term: its 16 values of the contraction are a quarter of a 128-byte row of the tile.
             const int j = j0 + rot < supers ? j0 + rot : j0 + rot - supers;
@@ -1108,7 +1101,7 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
             const int j = un >> 1, half = un & 1, sc = j % CST;
             ok = spl_mbar_wait(&full_c[sc], (j / CST) & 1, abort);
             if (!ok) { if (!*abort && lane == 0) spl_note_wait(error_flag, 41, un); break; }
-            const int n = PAIR ? 2 * half + min(GPS, g_count - j * GPS) : min(SPL_TC_SUPER, g_count - j * SPL_TC_SUPER);      // code groups of the stage up to this unit's last; the unit has those from 2 * half (the pair form: tile `half`'s two)
+            const int n = 2 * half + min(GPS, g_count - j * GPS);      // code groups of the stage up to this unit's last: the unit has those from 2 * half, tile `half`'s two
             // The unit's codes and scale/bias words are read before anything is converted, so the codes can be handed back at once.
             uint4 lo[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)}, hi[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
             uint32_t sbw[2] = {0u, 0u};
@@ -1149,8 +1142,8 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
 #pragma unroll
                         for (int w = 0; w < 4; ++w)
                             asm("{\n .reg .b32 xa, xb, xc, xd;\n"
-                                " shl.b32 xa, %4, 6;\n shl.b32 xb, %4, 2;\n shr.b32 xc, %4, 2;\n shr.b32 xd, %4, 6;\n"
-                                " lop3.b32 xa, xa, 0x03C003C0, 0x4C004C00, 0xEA;\n"
+                                " shr.b32 xb, %4, 4;\n prmt.b32 xc, %4, 0, 0x0321;\n shl.b32 xd, %4, 4;\n"
+                                " lop3.b32 xa, %4, 0x03C003C0, 0x4C004C00, 0xEA;\n"
                                 " lop3.b32 xb, xb, 0x03C003C0, 0x4C004C00, 0xEA;\n"
                                 " lop3.b32 xc, xc, 0x03C003C0, 0x4C004C00, 0xEA;\n"
                                 " lop3.b32 xd, xd, 0x03C003C0, 0x4C004C00, 0xEA;\n"
@@ -1163,9 +1156,8 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
                 }
             }
             // The unit's share of the second-term operand sits at its place among the stage's sixteen values; the rest is zero.
-            // (The pair form's stage is two groups of the contraction: they are the first or the second half of their four.)
-            int place = half;
-            if (PAIR) { const int jsrc = j + rot < supers ? j + rot : j + rot - supers; place = ((g_first + jsrc * GPS) >> 1) & 1; }
+            // (A stage is two groups of the contraction: they are the first or the second half of their four.)
+            const int jsrc = j + rot < supers ? j + rot : j + rot - supers, place = ((g_first + jsrc * GPS) >> 1) & 1;
             if (place == 0) { spl_tc_st4(tmem_aq + lane_base + slot * 8, aq[0], aq[1], aq[2], aq[3]); spl_tc_st4(tmem_aq + lane_base + slot * 8 + 4, 0u, 0u, 0u, 0u); }
             else { spl_tc_st4(tmem_aq + lane_base + slot * 8, 0u, 0u, 0u, 0u); spl_tc_st4(tmem_aq + lane_base + slot * 8 + 4, aq[0], aq[1], aq[2], aq[3]); }
             spl_tc_st_wait();
@@ -1195,9 +1187,9 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
         float *stage = reinterpret_cast<float *>(b_ring);       // [RN][128] fp32
         // The pair form holds two tiles' sums, one per issuing warp's accumulator: the output stage runs once for each.
 #pragma unroll 1
-        for (int om = 0; om < (PAIR ? 2 : 1); ++om) {
-        const int otile = PAIR ? (om ? tile1 : tile0) : tile;
-        if (PAIR && om == 1 && !has1) break;
+        for (int om = 0; om < 2; ++om) {
+        const int otile = om ? tile1 : tile0;
+        if (om == 1 && !has1) break;
         if (ok) {
             spl_tc_fence_after();
             const int n = otile * 128 + col;
@@ -1209,13 +1201,10 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
             for (int cb = set; cb < RN / 16; cb += SPL_TC_SETS) {
                 const int c0 = cb * 16;
                 float total[16];
+uint32_t v[16];
+                spl_tc_ld16(v, tmem_d + lane_base + om * RN + c0);
 #pragma unroll
-                for (int a = 0; a < (!PAIR && units > 1 ? 2 : 1); ++a) {
-                    uint32_t v[16];
-                    spl_tc_ld16(v, tmem_d + lane_base + (PAIR ? om : a) * RN + c0);
-#pragma unroll
-                    for (int r = 0; r < 16; ++r) total[r] = a == 0 ? __uint_as_float(v[r]) : total[r] + __uint_as_float(v[r]);
-                }
+                for (int r = 0; r < 16; ++r) total[r] = __uint_as_float(v[r]);
                 // A cut tile's partial sums are scaled one by one, so their sum is.
                 if (in_squares)
 #pragma unroll
@@ -1264,7 +1253,7 @@ spl_gemm_q4_narrow_kernel(const uint32_t *__restrict__ codes, const uint32_t *__
                     if ((t & 7) == 0) act_out.put_sum(row, otile, sa + sb2);
                 }
             }
-            if (PAIR) spl_named_barrier<1, SPL_TC_SETS * 128>();      // the staged sums have been read: the other tile's may follow
+            spl_named_barrier<1, SPL_TC_SETS * 128>();      // the staged sums have been read: the other tile's may follow
         }
         }
     }
@@ -1332,7 +1321,7 @@ __global__ void __launch_bounds__(256) spl_gemm_fixup_kernel(const float *__rest
     }
 }
 
-// The same for the narrow block's partial sums, partials[split][row][column] in the output's own columns: a warp per
+// The same for the pair form's partial sums, partials[split][row][column] in the output's own columns: a warp per
 // (row, 64 columns).
 __global__ void __launch_bounds__(256) spl_gemm_fixup_rows_kernel(const float *__restrict__ partials, int splits, int rows_padded, int rows, int ld,
                                                                   const float *residual, float *out, const uint16_t *__restrict__ emit_weight, SplOperand emit_out, float *emit_squares) {

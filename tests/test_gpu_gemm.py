@@ -58,6 +58,15 @@ def test_short_contractions_with_odd_stage_counts(oracle, k, rows):
     case(oracle, 384, k, rows, 100 + k)
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("n,k", [(19216, 512), (200, 2048), (384, 8960), (2064, 1280)])
+def test_row_edges_over_one_and_several_tiles_a_block_and_cut_tiles(oracle, n, k, rows):
+    """The kernels of up to 64 rows at the edges of their row counts: more tiles than SMs (151: some blocks take a second tile behind their first, the
+    last one 16 columns wide), two and three tiles cut in eight pieces of whole and of unequal length (35 stages of four groups), an odd tile count. Both
+    sides' sums are of exact fp32 terms; TOL is their order's, as above."""
+    case(oracle, n, k, rows, n + k + rows, residual=rows % 2 == 0)
+
+
 @pytest.mark.parametrize("n,k", [(17408, 5120), (5120, 17408), (10240, 5120), (5120, 6144)])
 def test_27b_shapes_at_64_rows(oracle, n, k):
     case(oracle, n, k, 64, 7)
