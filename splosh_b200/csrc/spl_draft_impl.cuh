@@ -136,13 +136,7 @@ static spl_status draft_linear(spl_draft *d, const uint16_t *bf16, int rows, int
     spl_tensor *t = new spl_tensor;
     spl_status s = alloc_q4(e, t->q, rows, inner);
     if (s == SPL_OK) s = upload_q4_into(e, t->q, 0, rows, inner, packed.data(), scales.data(), biases.data(), false);
-    size_t need = 0;
-    need = std::max(need, gemm_slot_floats(t->q, e->sms, 128, std::max(1, e->c.max_rows / 128), false, false));
-    if (s == SPL_OK && need > e->slot_floats) {
-        cudaFree(e->slots); e->slots = nullptr;
-        if (cudaMalloc(reinterpret_cast<void **>(&e->slots), need * 4) != cudaSuccess) s = e->fail(SPL_ERR_ALLOCATION_FAILED, "GEMM scratch");
-        else e->slot_floats = need;
-    }
+    if (s == SPL_OK) s = reserve_gemm_slots(e, t->q);
     if (s != SPL_OK) { cudaFree(t->q.codes); cudaFree(t->q.sb); delete t; return s; }
     *out = t;
     return SPL_OK;

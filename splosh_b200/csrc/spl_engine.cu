@@ -1963,6 +1963,19 @@ static __global__ void spl_silu_mul_kernel(float *gate, const float *__restrict_
         gate[i] = spl_bf16_to_float(spl_float_to_bf16(spl_silu_exact(gate[i]) * up[i]));
 }
 
+// The GEMM's scratch for partial sums has to hold those of a tensor of the caller's at any row count the engine takes, the last row block a part of one
+// (fewer row blocks may be cut in more pieces, so every count is asked). What is there is kept when there is no memory for more.
+static spl_status reserve_gemm_slots(spl_engine *e, const SplQ4Dev &w) {
+    size_t need = 0;
+    for (int row_blocks = 1; row_blocks <= e->rows_padded / 128; ++row_blocks) need = std::max(need, gemm_slot_floats(w, e->sms, 128, row_blocks, false, false));
+    if (need <= e->slot_floats) return SPL_OK;
+    float *more = nullptr;
+    if (cudaMalloc(reinterpret_cast<void **>(&more), need * 4) != cudaSuccess) { cudaGetLastError(); return e->fail(SPL_ERR_ALLOCATION_FAILED, "GEMM scratch"); }
+    cudaFree(e->slots);          // waits for the passes that use it
+    e->slots = more; e->slot_floats = need;
+    return SPL_OK;
+}
+
 spl_status spl_tensor_create_q4(spl_engine *e, int32_t rows, int32_t inner, const uint32_t *packed, const uint16_t *scales, const uint16_t *biases, spl_tensor **out) {
     if (!e || !packed || !scales || !biases || !out || rows <= 0 || inner <= 0 || inner % 256) return SPL_ERR_INVALID_ARGUMENT;
     SPL_NOT_IN_FLIGHT(e);
@@ -1971,15 +1984,7 @@ spl_status spl_tensor_create_q4(spl_engine *e, int32_t rows, int32_t inner, cons
     spl_tensor *t = new spl_tensor;
     spl_status s = alloc_q4(e, t->q, rows, inner);
     if (s == SPL_OK) s = upload_q4_into(e, t->q, 0, rows, inner, packed, scales, biases, false);
-    // The GEMM's scratch for partial sums has to hold this tensor's at any row count.
-    size_t need = 0;
-    const int row_blocks = std::max(1, e->c.max_rows / 128);
-    for (int rbs = 1; rbs <= row_blocks; ++rbs) need = std::max(need, gemm_slot_floats(t->q, e->sms, 128, rbs, false, false));
-    if (s == SPL_OK && need > e->slot_floats) {
-        cudaFree(e->slots); e->slots = nullptr;
-        if (cudaMalloc(reinterpret_cast<void **>(&e->slots), need * 4) != cudaSuccess) s = e->fail(SPL_ERR_ALLOCATION_FAILED, "GEMM scratch");
-        else e->slot_floats = need;
-    }
+    if (s == SPL_OK) s = reserve_gemm_slots(e, t->q);
     if (s != SPL_OK) { cudaFree(t->q.codes); cudaFree(t->q.sb); delete t; return s; }
     *out = t;
     return SPL_OK;

@@ -101,3 +101,23 @@ def test_the_primitives_refuse_what_they_cannot_hold(setup):
     with pytest.raises(S.EngineError):
         engine.pass_gemm(t, x.data_ptr(), 80, out.data_ptr())      # more rows than the engine's max_rows
     engine.tensor_destroy(t)
+
+
+@pytest.mark.parametrize("max_rows,rows", [(160, 130), (200, 200), (300, 129), (300, 300)])
+def test_row_counts_up_to_a_limit_that_is_no_multiple_of_128(max_rows, rows):
+    """A tensor whose contraction is cut leaves partial sums for every row block, the last one a part of 128 rows: the scratch that is set aside when the
+    tensor is created has to hold them at any row count up to the engine's limit."""
+    engine = S.Engine(S.tiny_geometry(), S.EngineConfig(max_slots=1, max_rows=max_rows, kv_pages=4, max_context=512))
+    rng = np.random.default_rng(rows)
+    n, inner = 2064, 2816
+    packed, scales, biases = O.quantize_mlx4((rng.standard_normal((n, inner)) * 0.02).astype(np.float32))
+    x = rng.standard_normal((rows, inner)).astype(np.float32)
+    tensor, dx, dout = engine.tensor_q4(packed, scales, biases), device(x), torch.empty((rows, n), device="cuda")
+    torch.cuda.synchronize()
+    engine.pass_begin()
+    engine.pass_gemm(tensor, dx.data_ptr(), rows, dout.data_ptr())
+    engine.pass_wait()
+    want = O.gemm_q4(packed, scales, biases, x)
+    assert np.abs(dout.cpu().numpy() - want).max() <= 8e-6 * np.abs(want).max()
+    engine.tensor_destroy(tensor)
+    engine.close()
