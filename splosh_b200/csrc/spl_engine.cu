@@ -343,6 +343,7 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
         n.act = reinterpret_cast<const unsigned char *>(op.values); n.means = reinterpret_cast<const unsigned char *>(op.sums);
         n.out = out; n.residual = residual; n.out_ld = w.ld; n.rows = rows; n.groups = w.k / 64; n.tiles = w.tiles; n.splits = splits;
         n.interleave = w.interleave; n.fuse = a.fuse; n.drop = g_drop_weight_stage; n.error_flag = scratch.error_flag;
+        n.wide = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 7) == 0;
         n.in_squares = x.in_squares; n.in_groups = x.in_dim / 64; n.in_dim = float(x.in_dim); n.eps = x.eps;
         n.act_out = a.act_out; n.emit_weight = x.emit_weight; n.emit_out = emit_out; n.emit_squares = x.emit_squares;
         cudaLaunchConfig_t cfg = {};

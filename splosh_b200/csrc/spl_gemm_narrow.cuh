@@ -35,6 +35,7 @@ struct SplNarrowArgs {
     float *out;
     const float *residual;
     int out_ld, rows, groups, tiles, splits, interleave, fuse, drop;
+    int wide;                              // out and residual lie on 8-byte boundaries (a caller's may lie on any float): two columns an access
     int *error_flag;
     const float *in_squares; int in_groups; float in_dim, eps;
     SplOperand act_out;                    // fuse: the SiLU-gated activation, the next GEMM's operand
@@ -70,6 +71,15 @@ __device__ __forceinline__ float2 spl_cluster_load2(uint32_t addr) {
     float2 v;
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
     return v;
+}
+
+// Two neighbouring columns of the output or the residual.
+__device__ __forceinline__ float2 spl_columns_load(const float *p, bool wide) {
+    return wide ? *reinterpret_cast<const float2 *>(p) : make_float2(p[0], p[1]);
+}
+__device__ __forceinline__ void spl_columns_store(float *p, float2 v, bool wide) {
+    if (wide) *reinterpret_cast<float2 *>(p) = v;
+    else { p[0] = v.x; p[1] = v.y; }
 }
 
 // What follows a tile's sum, by all converting warps of the blocks that hold its pieces: the pieces' sums are added in the order of the contraction
@@ -140,10 +150,10 @@ __device__ __forceinline__ void spl_narrow_output(const SplNarrowArgs &a, const 
             if (a.interleave > 0) { const int e = tile * 64 + (c2 >> 5) * 16 + (c2 & 15); n = ((c2 & 16) ? a.interleave : 0) + e; inside = e < a.interleave && row < a.rows; }
             if (inside) {
                 if (a.residual) {
-                    const float2 rv = a.interleave > 0 || k0 > 0 ? *reinterpret_cast<const float2 *>(a.residual + size_t(row) * a.out_ld + n) : res[k];
+                    const float2 rv = a.interleave > 0 || k0 > 0 ? spl_columns_load(a.residual + size_t(row) * a.out_ld + n, a.wide) : res[k];
                     x[k].x += rv.x; x[k].y += rv.y;
                 }
-                *reinterpret_cast<float2 *>(a.out + size_t(row) * a.out_ld + n) = x[k];
+                spl_columns_store(a.out + size_t(row) * a.out_ld + n, x[k], a.wide);
             } else x[k] = make_float2(0.0f, 0.0f);
             if (a.emit_weight) {
                 // The output feeds a deferred norm (Sources/Shaders/engine_na.metal:365-415): bf16(x * w) as the next operand, its per-64 sum, and the
@@ -410,7 +420,7 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
         for (int k = 0; k < PRE; ++k) {
             const int item = split * WARPS + warp + k * WARPS * S, row = item >> 1, n = tile * 128 + (item & 1) * 64 + 2 * lane;
             res[k] = make_float2(0.0f, 0.0f);
-            if (a.residual && a.interleave == 0 && row < a.rows && n < a.out_ld) res[k] = *reinterpret_cast<const float2 *>(a.residual + size_t(row) * a.out_ld + n);
+            if (a.residual && a.interleave == 0 && row < a.rows && n < a.out_ld) res[k] = spl_columns_load(a.residual + size_t(row) * a.out_ld + n, a.wide);
         }
         spl_named_barrier<1, SETS * 128>();
         if (ok && !spl_mbar_wait_warp(finished, t & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 40, t); }

@@ -121,3 +121,27 @@ def test_row_counts_up_to_a_limit_that_is_no_multiple_of_128(max_rows, rows):
     assert np.abs(dout.cpu().numpy() - want).max() <= 8e-6 * np.abs(want).max()
     engine.tensor_destroy(tensor)
     engine.close()
+
+
+@pytest.mark.parametrize("rows", [1, 24, 64])
+@pytest.mark.parametrize("n,inner", [(2064, 1280), (384, 1024), (1024, 2816)])
+def test_outputs_and_residuals_on_any_float_boundary(setup, n, inner, rows):
+    """A caller's output and residual may begin at any float: here one float past a 16-byte boundary, for a tensor of whole tiles and for ones whose
+    contraction is cut. Both sides add exact fp32 terms in another order: 8e-6 of the largest output, as everywhere for this GEMM. The floats around
+    the output stay as they were."""
+    _, _, engine = setup
+    rng = np.random.default_rng(n + inner + rows)
+    packed, scales, biases = O.quantize_mlx4((rng.standard_normal((n, inner)) * 0.02).astype(np.float32))
+    x, res = rng.standard_normal((rows, inner)).astype(np.float32), rng.standard_normal((rows, n)).astype(np.float32)
+    want = O.gemm_q4(packed, scales, biases, x, res)
+    tensor, dx = engine.tensor_q4(packed, scales, biases), device(x)
+    dres, dout = torch.zeros(rows * n + 4, device="cuda"), torch.full((rows * n + 4,), 7.0, device="cuda")
+    dres[1:1 + rows * n] = torch.from_numpy(res.reshape(-1)).cuda()
+    torch.cuda.synchronize()
+    engine.pass_begin()
+    engine.pass_gemm(tensor, dx.data_ptr(), rows, dout.data_ptr() + 4, dres.data_ptr() + 4)
+    engine.pass_wait()
+    got = dout.cpu().numpy()
+    assert (got[:1] == 7.0).all() and (got[1 + rows * n:] == 7.0).all()
+    assert np.abs(got[1:1 + rows * n].reshape(rows, n) - want).max() <= 8e-6 * np.abs(want).max()
+    engine.tensor_destroy(tensor)
