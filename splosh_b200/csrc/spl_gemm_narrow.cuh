@@ -42,6 +42,8 @@ struct SplNarrowArgs {
     const uint16_t *emit_weight; SplOperand emit_out; float *emit_squares;
 };
 
+// The barriers of this kernel, a block's and a cluster's, are instructions of whole converged warps (.aligned): where a warp has branched by lane since it last
+// met, a __syncwarp stands in front of them. Nothing else promises that its lanes have come together again.
 // A part in a barrier of the block without waiting for it.
 template <int ID, int COUNT> __device__ __forceinline__ void spl_named_arrive() { asm volatile("bar.arrive %0, %1;\n" ::"n"(ID), "n"(COUNT) : "memory"); }
 // K-major without swizzle: core matrices of eight rows of 16 bytes, `k_step` bytes from the first eight of a k16 to the last eight, 128 from eight rows to the next.
@@ -228,6 +230,7 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
         spl_named_arrive<2, SPL_NARROW_THREADS>();
     } else {
         spl_tc_fence_before();
+        __syncwarp();
         spl_named_barrier<2, SPL_NARROW_THREADS>();
         spl_tc_fence_after();
         spl_named_arrive<3, SPL_NARROW_THREADS>();
@@ -249,7 +252,7 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
             const unsigned char *src = (lane == 0 ? a.codes : a.sb) + (size_t(tile) * stages_all + s_first) * bytes;
             const int rot = rotation(tile);
             for (int i = 0; i < stages; ++i, ++n) {
-                if (n == CST) { spl_named_barrier<3, SPL_NARROW_THREADS>(); spl_grid_begin(); }
+                if (n == CST) { __syncwarp(); spl_named_barrier<3, SPL_NARROW_THREADS>(); spl_grid_begin(); }
                 if (n >= CST) ok = spl_mbar_wait_warp(&empty_c[slot], parity, abort);
                 if (!ok) { if (!*abort && lane == 0) spl_note_wait(a.error_flag, 10, i); break; }
                 issued_c = n + 1;
@@ -261,7 +264,7 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
                 if (++slot == CST) { slot = 0; parity ^= 1u; }
             }
         }
-        if (n <= CST && ok) { spl_named_barrier<3, SPL_NARROW_THREADS>(); spl_grid_begin(); }
+        if (n <= CST && ok) { __syncwarp(); spl_named_barrier<3, SPL_NARROW_THREADS>(); spl_grid_begin(); }
     } else if (warp == W_COPYB) {
         // ---- copies of activations (lane 0) and of their split means (lane 1), a stage at a time; a lane each waits for one of the units that had the place.
         {
@@ -422,6 +425,7 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
             res[k] = make_float2(0.0f, 0.0f);
             if (a.residual && a.interleave == 0 && row < a.rows && n < a.out_ld) res[k] = spl_columns_load(a.residual + size_t(row) * a.out_ld + n, a.wide);
         }
+        __syncwarp();
         spl_named_barrier<1, SETS * 128>();
         if (ok && !spl_mbar_wait_warp(finished, t & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 40, t); }
         if (ok && set * 16 < RN) {
@@ -440,8 +444,10 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
         }
         __syncwarp();
         if (lane == 0) spl_mbar_arrive(drained);
+        __syncwarp();
         if (S > 1) { spl_cluster_barrier(); } else spl_named_barrier<1, SETS * 128>();
         if (!*abort) spl_narrow_output<RN>(a, plane, tile, split, S, warp, lane, res);
+        __syncwarp();
         if (S == 1) spl_named_barrier<1, SETS * 128>();        // the sums have been read: the next tile's may come
         }
     }
