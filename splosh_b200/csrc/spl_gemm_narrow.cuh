@@ -11,8 +11,8 @@
 //     a converting set answers for the activations, so an issuing warp waits once a unit;
 //   * waits that are nearly always over are asked about ahead (mbarrier.test_wait) and looked at after other work;
 //   * of a block's 27K cycles 9K were set-up, first copies and output. Blocks of tiles that are not cut stay and take the next tile, whose weights are
-//     on their way while a tile's sums are written; nobody waits for the copier's first copies any more; output items are
-//     taken several at a time, everything they need asked for first.
+//     on their way while a tile's sums are written; nobody waits for the copier's first copies any more; the SiLU
+//     gate's rows are taken several at a time, everything they need asked for first, and what the other outputs need is asked for before the sums are there.
 // The blocks of a cut tile are a cluster: the cluster's warps add the blocks' sums through distributed shared memory and write the output, with the
 // residual and the next deferred norm's operand. (They used to leave partial sums in global memory for a second kernel.)
 // Measured before and after, with those second kernels: gate|up (34,816 x 5,120) at 16 rows 34.8 -> 28 us, out and down together 16.5 -> 13.5 us a launch; a
@@ -84,13 +84,18 @@ __device__ __forceinline__ void spl_columns_store(float *p, float2 v, bool wide)
     else { p[0] = v.x; p[1] = v.y; }
 }
 
-// What follows a tile's sum, by all converting warps of the blocks that hold its pieces: the pieces' sums are added in the order of the contraction
-// (through distributed shared memory where a tile is cut). A warp takes PRE items at a time and asks for everything they need before it works on any.
+// A converting thread's two columns of its warp's output items, and what they need that can be asked for before the sums are there: the residual of the
+// first item, the weight of the next norm.
+struct SplNarrowColumns { int n; bool inside; float2 res; uint32_t weight; };
+
+// What follows a tile's sum where a row's columns have to meet (SiLU gate, next operand) or the tile is cut, by all converting warps of the blocks that hold its pieces: the pieces' sums are added in the order of the contraction
+// (through distributed shared memory where a tile is cut).
 template <int RN>
-__device__ __forceinline__ void spl_narrow_output(const SplNarrowArgs &a, const float *plane, int tile, int split, int S, int warp, int lane, const float2 (&res)[RN / 16]) {
-    constexpr int PRE = RN / 16, WARPS = SPL_TC_SETS * 4;
-    const uint32_t base = spl_smem_addr(plane);
+__device__ __forceinline__ void spl_narrow_output(const SplNarrowArgs &a, const float *plane, int tile, int split, int S, int warp, int lane, const SplNarrowColumns &at) {
+    constexpr int WARPS = SPL_TC_SETS * 4;
     if (a.fuse) {
+        constexpr int PRE = RN / 16;          // rows a warp takes at a time, everything asked for before any is worked on
+        const uint32_t base = spl_smem_addr(plane);
         // A fused gate|up tensor: in each run of 32 columns of a tile the first sixteen are gate columns and the next sixteen the up columns of the same
         // elements. act = bf16(silu(gate) * up) (Sources/Shaders/engine.metal:200-219) into the next GEMM's operand, a warp a row.
         const int e = 2 * lane, gc = (e >> 4) * 32 + (e & 15);
@@ -119,54 +124,46 @@ __device__ __forceinline__ void spl_narrow_output(const SplNarrowArgs &a, const 
         }
         return;
     }
+    // An item is a row's 64 columns, every WARPS x S-th of a tile's a warp's: all of the same half of the tile. What bounds this stage is instruction fetches
+    // and trips to the other blocks' memory. The body therefore stands here once (a block comes here once, and pays for every instruction's first use), a
+    // warp reads what it has items for and no more, and four blocks' sums are on their way at a time. Taking RN / 16 items at a time, the last one again where
+    // there were fewer, a block after the other: 1,024 x 5,120 at 64 rows 13.7 us with its operand, now 10.4; 128 x 4,096 13.3, now 9.0; 5,120 x 6,144 at one
+    // row 11.1, now 11.0, at 24 rows 12.2, now 11.7.
+    const int step = WARPS * S, n = at.n;
+    const uint32_t plane_at = spl_smem_addr(plane) + uint32_t((warp & 1) * 64 + 2 * lane) * 4;
+    float2 res = at.res;
 #pragma unroll 1
-    for (int k0 = 0; split * WARPS + warp + k0 * WARPS * S < a.rows * 2; k0 += PRE) {
-        float2 x[PRE];
-        uint32_t w2[PRE];
-#pragma unroll
-        for (int k = 0; k < PRE; ++k) {
-            const int item = split * WARPS + warp + (k0 + k) * WARPS * S, c2 = (item & 1) * 64 + 2 * lane;
-            x[k] = make_float2(0.0f, 0.0f);
-            w2[k] = (a.emit_weight && tile * 128 + c2 < a.out_ld) ? *reinterpret_cast<const uint32_t *>(a.emit_weight + tile * 128 + c2) : 0u;
-        }
-        const uint32_t at = base + uint32_t(warp * 64 + 2 * lane) * 4;          // the items of a warp are WARPS x S / 2 rows apart, all of the same half
+    for (int item = split * WARPS + warp; item < a.rows * 2; item += step) {
+        const int row = item >> 1;
+        float2 next = make_float2(0.0f, 0.0f);
+        if (a.residual && at.inside && item + step < a.rows * 2) next = spl_columns_load(a.residual + size_t(row + step / 2) * a.out_ld + n, a.wide);
+        // The pieces' sums in the order of the contraction, four blocks asked at a time.
+        float2 x = make_float2(0.0f, 0.0f);
 #pragma unroll 1
-        for (int r = 0; r < S; ++r) {
-            if (S == 1) {
+        for (int r0 = 0; r0 < S; r0 += 4) {
+            if (S == 1) { x = spl_shared_load2(plane_at + uint32_t(row) * 512); break; }
+            float2 p[4];
 #pragma unroll
-                for (int k = 0; k < PRE; ++k) x[k] = spl_shared_load2(at + uint32_t(min((k0 + k) * WARPS, RN * 2 - WARPS)) * 256);
-                break;
-            }
-            const uint32_t from = spl_cluster_map(at, r);
+            for (int r = 0; r < 4; ++r)
+                if (r0 + r < S) p[r] = spl_cluster_load2(spl_cluster_map(plane_at + uint32_t(row) * 512, r0 + r));
 #pragma unroll
-            for (int k = 0; k < PRE; ++k) {
-                const float2 p = spl_cluster_load2(from + uint32_t(min(split * WARPS + (k0 + k) * WARPS * S, RN * 2 - WARPS)) * 256);
-                x[k] = r == 0 ? p : make_float2(x[k].x + p.x, x[k].y + p.y);
-            }
+            for (int r = 0; r < 4; ++r)
+                if (r0 + r < S) x = r0 + r == 0 ? p[r] : make_float2(x.x + p[r].x, x.y + p[r].y);
         }
-#pragma unroll
-        for (int k = 0; k < PRE; ++k) {
-            const int item = split * WARPS + warp + (k0 + k) * WARPS * S, row = item >> 1, half = item & 1, c2 = half * 64 + 2 * lane;
-            int n = tile * 128 + c2;
-            bool inside = n < a.out_ld && row < a.rows;
-            if (a.interleave > 0) { const int e = tile * 64 + (c2 >> 5) * 16 + (c2 & 15); n = ((c2 & 16) ? a.interleave : 0) + e; inside = e < a.interleave && row < a.rows; }
-            if (inside) {
-                if (a.residual) {
-                    const float2 rv = a.interleave > 0 || k0 > 0 ? spl_columns_load(a.residual + size_t(row) * a.out_ld + n, a.wide) : res[k];
-                    x[k].x += rv.x; x[k].y += rv.y;
-                }
-                spl_columns_store(a.out + size_t(row) * a.out_ld + n, x[k], a.wide);
-            } else x[k] = make_float2(0.0f, 0.0f);
-            if (a.emit_weight) {
-                // The output feeds a deferred norm (Sources/Shaders/engine_na.metal:365-415): bf16(x * w) as the next operand, its per-64 sum, and the
-                // squares of x per 64 columns. Both sums are butterflies over the warp: one fixed order.
-                const float v0 = spl_bf16_to_float(spl_float_to_bf16(x[k].x * spl_bf16_to_float(uint16_t(w2[k] & 0xFFFFu))));
-                const float v1 = spl_bf16_to_float(spl_float_to_bf16(x[k].y * spl_bf16_to_float(uint16_t(w2[k] >> 16))));
-                if (inside) *reinterpret_cast<__half2 *>(reinterpret_cast<__half *>(a.emit_out.values) + a.emit_out.at(row, n)) = __halves2half2(__float2half_rn(v0), __float2half_rn(v1));
-                const float vs = spl_warp_sum(v0 + v1), sq = spl_warp_sum(x[k].x * x[k].x + x[k].y * x[k].y);
-                const int group = tile * 2 + half;
-                if (lane == 0 && row < a.rows && group * 64 < a.out_ld) { a.emit_out.put_sum(row, group, vs); a.emit_squares[size_t(row) * (a.out_ld / 64) + group] = sq; }
-            }
+        if (at.inside) {
+            if (a.residual) { x.x += res.x; x.y += res.y; }
+            spl_columns_store(a.out + size_t(row) * a.out_ld + n, x, a.wide);
+        } else x = make_float2(0.0f, 0.0f);
+        res = next;
+        if (a.emit_weight) {
+            // The output feeds a deferred norm (Sources/Shaders/engine_na.metal:365-415): bf16(x * w) as the next operand, its per-64 sum, and the
+            // squares of x per 64 columns. Both sums are butterflies over the warp: one fixed order.
+            const float v0 = spl_bf16_to_float(spl_float_to_bf16(x.x * spl_bf16_to_float(uint16_t(at.weight & 0xFFFFu))));
+            const float v1 = spl_bf16_to_float(spl_float_to_bf16(x.y * spl_bf16_to_float(uint16_t(at.weight >> 16))));
+            if (at.inside) *reinterpret_cast<__half2 *>(reinterpret_cast<__half *>(a.emit_out.values) + a.emit_out.at(row, n)) = __halves2half2(__float2half_rn(v0), __float2half_rn(v1));
+            const float vs = spl_warp_sum(v0 + v1), sq = spl_warp_sum(x.x * x.x + x.y * x.y);
+            const int group = tile * 2 + (warp & 1);
+            if (lane == 0 && group * 64 < a.out_ld) { a.emit_out.put_sum(row, group, vs); a.emit_squares[size_t(row) * (a.out_ld / 64) + group] = sq; }
         }
     }
 }
@@ -195,6 +192,7 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int W_COPY = WARPS, W_MMA0 = W_COPY + 1, W_COPYB = W_COPY + 2, W_MMA1 = W_COPY + 3;
+    const bool direct = a.splits == 1 && !a.fuse && !a.emit_weight;
     const int S = a.splits, split = S == 1 ? 0 : int(blockIdx.x) % S, tile0 = S == 1 ? int(blockIdx.x) : int(blockIdx.x) / S, tile_step = S == 1 ? int(gridDim.x) : a.tiles;
     const int stages_all = a.groups / SG, per = S == 1 ? stages_all : (stages_all + S - 1) / S, s_first = split * per, stages = min(per, stages_all - s_first), units = 2 * stages;
     // Every block of a GEMM reads the same activation lines. Blocks therefore walk the contraction from different starting points (a fixed function
@@ -239,7 +237,6 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
     // Two accumulators of RN columns, one per issuing warp; the operand slots; the second terms' operands.
     const uint32_t tmem_d = tmem, tmem_a = tmem + 128, tmem_aq = tmem_a + AUN * 64;
     bool ok = true;
-    constexpr int PRE = RN / 16;          // output items a warp takes at a time
     int issued_c = 0, issued_b = 0;
     if (warp == W_COPY) {
         // ---- copies of the weight: lane 0 the codes, lane 1 the scale/bias words. They are nobody's output: the ring is filled before the wait for the
@@ -418,12 +415,16 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
                 if (lane == 0) row_factor[warp + 16 * f] = 1.0f / sqrtf(ss / a.in_dim + a.eps);
             }
         // A load asked for now comes while the last products are formed.
-        float2 res[PRE];
-#pragma unroll
-        for (int k = 0; k < PRE; ++k) {
-            const int item = split * WARPS + warp + k * WARPS * S, row = item >> 1, n = tile * 128 + (item & 1) * 64 + 2 * lane;
-            res[k] = make_float2(0.0f, 0.0f);
-            if (a.residual && a.interleave == 0 && row < a.rows && n < a.out_ld) res[k] = spl_columns_load(a.residual + size_t(row) * a.out_ld + n, a.wide);
+        SplNarrowColumns at = {tile * 128 + (warp & 1) * 64 + 2 * lane, false, make_float2(0.0f, 0.0f), 0u};
+        at.inside = at.n < a.out_ld;
+        if (a.interleave > 0) {
+            const int c2 = (warp & 1) * 64 + 2 * lane, e = tile * 64 + (c2 >> 5) * 16 + (c2 & 15);
+            at.n = ((c2 & 16) ? a.interleave : 0) + e; at.inside = e < a.interleave;
+        }
+        {
+            const int row = (split * WARPS + warp) >> 1;
+            if (a.residual && at.inside && row < a.rows) at.res = spl_columns_load(a.residual + size_t(row) * a.out_ld + at.n, a.wide);
+            if (a.emit_weight && at.inside) at.weight = *reinterpret_cast<const uint32_t *>(a.emit_weight + at.n);
         }
         __syncwarp();
         spl_named_barrier<1, SETS * 128>();
@@ -435,18 +436,39 @@ spl_gemm_q4_narrow_kernel(const __grid_constant__ SplNarrowArgs a) {
             spl_tc_ld16(v1, tmem_d + lane_base + RN + set * 16);
             spl_tc_fence_before();
             // A cut tile's partial sums are scaled one by one, so their sum is.
+            float x[16];
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
-                float x = __uint_as_float(v0[r]) + __uint_as_float(v1[r]);
-                if (a.in_squares) x *= row_factor[set * 16 + r];
-                plane[(set * 16 + r) * 128 + col] = x;
+                x[r] = __uint_as_float(v0[r]) + __uint_as_float(v1[r]);
+                if (a.in_squares) x[r] *= row_factor[set * 16 + r];
             }
+            if (direct) {
+                // A whole tile's plain output goes from the registers to its place, a column a thread (any float address will do): nobody else has to see
+                // it. Through the plane, as the other outputs go, 17,408 x 5,120 at 64 rows took 21.4 us with its operand, and takes 20.3.
+                const int e = tile * 64 + (col >> 5) * 16 + (col & 15), n = a.interleave > 0 ? ((col & 16) ? a.interleave : 0) + e : tile * 128 + col;
+                if (a.interleave > 0 ? e < a.interleave : n < a.out_ld) {
+                    const int last = a.rows - set * 16;
+                    const size_t first = size_t(set * 16) * a.out_ld + n;
+#pragma unroll
+                    for (int r0 = 0; r0 < 16; r0 += 4) {
+                        float res[4];
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) res[r] = a.residual && r0 + r < last ? a.residual[first + size_t(r0 + r) * a.out_ld] : 0.0f;
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+                            if (r0 + r < last) a.out[first + size_t(r0 + r) * a.out_ld] = a.residual ? __fadd_rn(x[r0 + r], res[r]) : x[r0 + r];
+                    }
+                }
+            } else
+#pragma unroll
+                for (int r = 0; r < 16; ++r) plane[(set * 16 + r) * 128 + col] = x[r];
         }
         __syncwarp();
         if (lane == 0) spl_mbar_arrive(drained);
+        if (direct) continue;
         __syncwarp();
         if (S > 1) { spl_cluster_barrier(); } else spl_named_barrier<1, SETS * 128>();
-        if (!*abort) spl_narrow_output<RN>(a, plane, tile, split, S, warp, lane, res);
+        if (!*abort) spl_narrow_output<RN>(a, plane, tile, split, S, warp, lane, at);
         __syncwarp();
         if (S == 1) spl_named_barrier<1, SETS * 128>();        // the sums have been read: the next tile's may come
         }
