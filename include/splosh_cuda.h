@@ -318,6 +318,9 @@ spl_status spl_debug_gdn_chunk_min(spl_engine *engine, int32_t rows);
 /* Tests: the launch of a GGUF GEMM of type `format` (12 Q4_K, 13 Q5_K, 14 Q6_K), `n` columns over `k`, for `rows` rows on a device of `sms` SMs, its
  * scratch unlimited: the rows of a block and the pieces its contraction is cut in. Host arithmetic, no device needed. */
 spl_status spl_debug_gguf_plan(int32_t format, int32_t n, int32_t k, int32_t rows, int32_t sms, int32_t *block_rows, int32_t *pieces);
+/* Tests: the pieces that the contraction of an MLX affine-4 GEMM of up to 64 rows, `n` columns over `k`, is cut in on a device of `sms` SMs that holds
+ * clusters[s - 1] clusters of s blocks at a time, s = 1 ... 8. Host arithmetic, no device needed. */
+spl_status spl_debug_q4_plan(int32_t n, int32_t k, int32_t sms, const int32_t *clusters, int32_t *pieces);
 /* Tests: the GGUF GEMMs of this engine's steps of more than 64 rows run in blocks of `rows` rows (64 or 128; 0, the default: by waves of blocks). */
 spl_status spl_debug_gguf_block_rows(spl_engine *engine, int32_t rows);
 /* Tests and measurements: with `enabled` 0 the GEMMs of steps of more than 64 rows run on the 128-row block that works on

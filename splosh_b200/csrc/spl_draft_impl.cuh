@@ -148,7 +148,7 @@ static spl_status draft_gemm_wide(spl_draft *d, const SplQ4Dev &w, const float *
     const int rn = operand_rn(rows), blocks = (rows + rn - 1) / rn;
     const SplOperand operand{d->wide_act, d->wide_sums, rn, blocks};
     launch_step(spl_operand_kernel, dim3(rows), dim3(256), 0, e->stream, in, operand, w.k);
-    const GemmScratch scratch{e->slots, e->slot_floats, e->tc_error, e->sms};
+    const GemmScratch scratch{e->slots, e->slot_floats, e->tc_error, e->sms, e->clusters};
     if (!launch_gemm_rows(e->stream, w, GemmOperand{d->wide_act, d->wide_sums, rn, blocks}, out, nullptr, rows, scratch, GemmExtras(), nullptr))
         return draft_fail(d, SPL_ERR_INVALID_ROWS, "the GEMM scratch is smaller than the context pass needs");
     return check_launch(e, "draft fc");

@@ -78,6 +78,7 @@ struct spl_engine {
     int gdn_chunk_min = SPL_GDN_CHUNK_MIN;      // ordinary runs at least this long take the chunked gated-delta scan (spl_debug_gdn_chunk_min)
     int gguf_block_rows = 0;      // test switch (spl_debug_gguf_block_rows)
     int sms = 148;
+    const int *clusters = nullptr;     // clusters of 1 ... SPL_NARROW_CLUSTER blocks of the narrow GEMM that are resident at a time (configure_device)
     int rows_padded = 0, logit_rows_padded = 0;
     int *tc_error = nullptr;
     // Drafter feature taps (Engine.swift:330-331, 1488-1497): the residual stream after the listed blocks, [row][tap][hidden].
@@ -226,8 +227,8 @@ struct GemmExtras {
     const float *in_squares = nullptr; int in_dim = 0; float eps = 0.0f;
     const uint16_t *emit_weight = nullptr; const SplOperand *emit_out = nullptr; float *emit_squares = nullptr;
 };
-// Where the blocks of a cut tile leave their partial sums, the launch's error words, the device's SM count.
-struct GemmScratch { float *slots; size_t slot_floats; int *error_flag; int sms; spl_engine *timed = nullptr; };    // timed: the engine whose profile times the second kernel as elementwise work
+// Where the blocks of a cut tile leave their partial sums, the launch's error words, the device's SM count and how many clusters of each size it holds.
+struct GemmScratch { float *slots; size_t slot_floats; int *error_flag; int sms; const int *clusters; spl_engine *timed = nullptr; };    // timed: the engine whose profile times the second kernel as elementwise work
 
 // The kernels that need more than the default shared memory, opted in on the current device (the attribute is per device).
 template <int RN> void configure_gemm() {
@@ -241,10 +242,10 @@ template <int RN> void configure_gemm() {
 }
 template <int RN, int FMT> void configure_gguf() { cudaFuncSetAttribute(spl_gemm_gguf_tc_kernel<RN, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_gguf_smem_bytes(RN, FMT))); }
 template <int HD, int PER_KV> void configure_scan() { cudaFuncSetAttribute(spl_attn_scan_kernel<HD, PER_KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(spl_attn_smem_bytes(HD, spl_attn_nq(PER_KV)))); }
-// Once per device and process, with that device current. `sms` (may be null) receives its SM count.
-bool configure_device(int device, int *sms) {
+// Once per device and process, with that device current. `sms` receives its SM count, `clusters` the counts that narrow_splits goes by.
+bool configure_device(int device, int *sms, const int **clusters) {
     static bool done[64] = {};
-    static int count[64] = {};
+    static int count[64] = {}, resident[64][SPL_NARROW_CLUSTER + 1] = {};
     if (device < 0 || device >= 64) return false;
     if (!done[device]) {
         configure_gemm<16>(); configure_gemm<32>(); configure_gemm<64>(); configure_gemm<128>();
@@ -258,34 +259,66 @@ bool configure_device(int device, int *sms) {
         cudaDeviceProp prop;
         if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return false;
         count[device] = prop.multiProcessorCount;
+        for (int s = 1; s <= SPL_NARROW_CLUSTER; ++s) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(s); cfg.blockDim = dim3(SPL_NARROW_THREADS); cfg.dynamicSmemBytes = spl_narrow_smem_bytes(64);
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr; cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&resident[device][s], spl_gemm_q4_narrow_kernel<64>, &cfg) != cudaSuccess) return false;
+        }
         if (cudaGetLastError() != cudaSuccess) return false;
         done[device] = true;
     }
-    if (sms) *sms = count[device];
+    *sms = count[device];
+    *clusters = resident[device];
     return true;
 }
 
-// How a GEMM's weight is cut in pieces, one block a piece and row block: every tile in `splits` pieces, the count that
-// minimises waves x stages per block with a fixed cost per block, and the second kernel of a cut GEMM, counted in.
-// `whole`: the block's output stage needs the whole sum (the fused SiLU gate), so tiles are not cut.
 // Test switch (spl_debug_drop_weight_stage): the q4 GEMM's weight-copy role leaves out this stage of every block's piece, so
 // the roles that wait for it run out of time. -1: off.
 static int g_drop_weight_stage = -1;
 // Test switch (spl_debug_pair_blocks): 0 keeps prompt chunks on the one-tile 128-row block.
 static int g_pair_blocks = 1;
 
+// How the one-tile 128-row block's weight is cut in pieces, one block a piece and row block: every tile in `splits` pieces, the count that
+// minimises waves x stages per block with a fixed cost per block, and the second kernel of a cut GEMM, counted in.
+// `whole`: the block's output stage needs the whole sum (the fused SiLU gate), so tiles are not cut.
 struct GemmCut { int pieces, splits; };
-GemmCut gemm_cut(const SplQ4Dev &w, int sms, int rn, int row_blocks, bool whole) {
-    const int stages = w.k / (64 * spl_tc_super(rn));
+GemmCut gemm_cut(const SplQ4Dev &w, int sms, int row_blocks, bool whole) {
+    const int stages = w.k / (64 * spl_tc_super(128));
     int best = 1; double best_cost = 1e30;
-    for (int s = 1; s <= stages && s <= (rn < 128 ? SPL_NARROW_CLUSTER : 16) && !(whole && s > 1); ++s) {
+    for (int s = 1; s <= stages && s <= 16 && !(whole && s > 1); ++s) {
         const int per = (stages + s - 1) / s;
         if (s > 1 && per < 2) break;
         const int waves = (w.tiles * s * row_blocks + sms - 1) / sms;
-        const double cost = double(waves) * (per * spl_tc_super(rn) + 20.0) + (s > 1 ? 12.0 : 0.0);      // in groups of time: a block's fill and output cost about twenty, the second kernel twelve
+        const double cost = double(waves) * (per * spl_tc_super(128) + 20.0) + (s > 1 ? 12.0 : 0.0);      // in groups of time: a block's fill and output cost about twenty, the second kernel twelve
         if (cost < best_cost - 1e-9) { best_cost = cost; best = s; }
     }
     return {w.tiles * best, best};
+}
+
+// Into how many pieces of whole stages the narrow block's tiles are cut (asked for `s`, it may be fewer: no piece is empty), by the same count. The blocks of a cut
+// tile are a cluster and have to find room in one GPC together, so what runs at a time is counted in clusters: 148 SMs hold 45 of three blocks, 26 of five,
+// 15 of seven. (Counted in blocks, 2,048 x 5,120 went in sixteen clusters of seven, one of them in a second wave: 14.8 us at one row and 25.2 at 64 with
+// its operand, where five pieces take 8.9 and 11.0.) A wave of clusters behind the first costs twelve more: a cluster waits until all its blocks have room.
+// Without that 12,288 x 17,408 went in three waves of fours, 51.0 us and 59.6, and is 49.0 and 51.8 uncut; 6,144 x 17,408 in two of fives, 29.9 and 39.5
+// (two pieces: 28.3, 34.3). The other constants are those of the 128-row block: they keep the cut, and so the order of the sums, of every tensor whose
+// clusters run in one wave.
+int narrow_splits(const SplQ4Dev &w, int sms, const int *clusters, bool whole) {
+    const int stages = w.k / 256;
+    int best = 1; double best_cost = 1e30;
+    for (int s = 1; s <= stages && s <= SPL_NARROW_CLUSTER && !(whole && s > 1); ++s) {
+        const int per = (stages + s - 1) / s, pieces = (stages + per - 1) / per;
+        if (s > 1 && per < 2) break;
+        if (pieces > 1 && clusters[pieces] < 1) continue;
+        int waves = (w.tiles * s + sms - 1) / sms;
+        if (pieces > 1) waves = std::max(waves, (w.tiles + clusters[pieces] - 1) / clusters[pieces]);
+        const double cost = double(waves) * (per * 4 + 20.0) + (s > 1 ? 12.0 * waves : 0.0);
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = pieces; }
+    }
+    return best;
 }
 
 // The pair form of the 128-row block (two tiles of the weight a block): into how many runs of whole stages every pair's
@@ -310,7 +343,7 @@ int pair_splits(const SplQ4Dev &w, int sms, int row_blocks, bool whole) {
 // partials[split][row][column] (cut tiles, and every tile when the output feeds a deferred norm: `emit`).
 size_t gemm_slot_floats(const SplQ4Dev &w, int sms, int rn, int row_blocks, bool emit, bool whole) {
     if (rn < 128) return 0;          // the blocks of the narrow kernel's cut tiles meet in a cluster
-    const GemmCut cut = gemm_cut(w, sms, rn, row_blocks, whole);
+    const GemmCut cut = gemm_cut(w, sms, row_blocks, whole);
     // The pair form leaves cut contractions, and an output that feeds a deferred norm, to the second kernel.
     const int ps = pair_splits(w, sms, row_blocks, whole);
     const size_t pair = (ps > 1 || (ps == 1 && emit)) ? size_t(ps) * row_blocks * rn * w.ld : 0;
@@ -320,32 +353,18 @@ size_t gemm_slot_floats(const SplQ4Dev &w, int sms, int rn, int row_blocks, bool
 template <int RN>
 bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &op, float *out, const float *residual, int rows,
                     const GemmScratch &scratch, const GemmExtras &x, int *launches) {
-    const int row_blocks = (rows + RN - 1) / RN;
-    const GemmCut cut = gemm_cut(w, scratch.sms, RN, row_blocks, x.fuse_act != nullptr);
-    if (RN >= 128 && spl_tc_slot_floats(cut.pieces, cut.splits, row_blocks, RN) > scratch.slot_floats) return false;
-    SplGemmArgs a = {};
-    a.codes = w.codes; a.sb = w.sb; a.act = op.values; a.act_sums = op.sums; a.out = out; a.residual = residual;
-    a.slots = scratch.slots; a.error_flag = scratch.error_flag;
-    a.out_ld = w.ld; a.rows = rows; a.op_blocks = op.blocks; a.tiles = w.tiles; a.stages_per_tile = w.k / (64 * spl_tc_super(RN)); a.interleave = w.interleave;
-    a.pieces = cut.pieces; a.row_blocks = row_blocks; a.splits = cut.splits;
-    a.drop_stage = g_drop_weight_stage;
-    a.fuse = x.fuse_act ? 1 : 0;
-    a.act_out = x.fuse_act ? *x.fuse_act : SplOperand{nullptr, nullptr, RN, 1};
-    a.in_squares = x.in_squares; a.in_groups = x.in_dim / 64; a.in_dim = float(x.in_dim); a.eps = x.eps;
-    const SplOperand emit_out = x.emit_out ? *x.emit_out : SplOperand{nullptr, nullptr, RN, 1};
-    a.emit_weight = x.emit_weight; a.emit_out = emit_out; a.emit_squares = x.emit_squares;
-    const dim3 grid(cut.pieces * row_blocks), block(SPL_TC_THREADS);
     if constexpr (RN < 128) {
         // The narrow block: a cut tile's pieces are a cluster of blocks, one tile a cluster; a block of an uncut tensor stays and takes every gridDim.x-th tile.
-        const int stages = w.k / 256, per = (stages + cut.splits - 1) / cut.splits, splits = (stages + per - 1) / per;
+        const int splits = narrow_splits(w, scratch.sms, scratch.clusters, x.fuse_act != nullptr);
         SplNarrowArgs n = {};
         n.codes = reinterpret_cast<const unsigned char *>(w.codes); n.sb = reinterpret_cast<const unsigned char *>(w.sb);
         n.act = reinterpret_cast<const unsigned char *>(op.values); n.means = reinterpret_cast<const unsigned char *>(op.sums);
         n.out = out; n.residual = residual; n.out_ld = w.ld; n.rows = rows; n.groups = w.k / 64; n.tiles = w.tiles; n.splits = splits;
-        n.interleave = w.interleave; n.fuse = a.fuse; n.drop = g_drop_weight_stage; n.error_flag = scratch.error_flag;
+        n.interleave = w.interleave; n.fuse = x.fuse_act ? 1 : 0; n.drop = g_drop_weight_stage; n.error_flag = scratch.error_flag;
         n.wide = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 7) == 0;
         n.in_squares = x.in_squares; n.in_groups = x.in_dim / 64; n.in_dim = float(x.in_dim); n.eps = x.eps;
-        n.act_out = a.act_out; n.emit_weight = x.emit_weight; n.emit_out = emit_out; n.emit_squares = x.emit_squares;
+        n.act_out = x.fuse_act ? *x.fuse_act : SplOperand{nullptr, nullptr, RN, 1};
+        n.emit_weight = x.emit_weight; n.emit_out = x.emit_out ? *x.emit_out : SplOperand{nullptr, nullptr, RN, 1}; n.emit_squares = x.emit_squares;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(splits > 1 ? w.tiles * splits : std::min(w.tiles, scratch.sms)); cfg.blockDim = dim3(SPL_NARROW_THREADS); cfg.dynamicSmemBytes = spl_narrow_smem_bytes(RN); cfg.stream = stream;
         cudaLaunchAttribute attr[2];
@@ -357,8 +376,22 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
         cudaLaunchKernelEx(&cfg, spl_gemm_q4_narrow_kernel<RN>, n);
         if (launches) ++*launches;
         return true;
-    }
-    if constexpr (RN == 128) {
+    } else {
+        const int row_blocks = (rows + RN - 1) / RN;
+        const GemmCut cut = gemm_cut(w, scratch.sms, row_blocks, x.fuse_act != nullptr);
+        if (spl_tc_slot_floats(cut.pieces, cut.splits, row_blocks, RN) > scratch.slot_floats) return false;
+        SplGemmArgs a = {};
+        a.codes = w.codes; a.sb = w.sb; a.act = op.values; a.act_sums = op.sums; a.out = out; a.residual = residual;
+        a.slots = scratch.slots; a.error_flag = scratch.error_flag;
+        a.out_ld = w.ld; a.rows = rows; a.op_blocks = op.blocks; a.tiles = w.tiles; a.stages_per_tile = w.k / (64 * spl_tc_super(RN)); a.interleave = w.interleave;
+        a.pieces = cut.pieces; a.row_blocks = row_blocks; a.splits = cut.splits;
+        a.drop_stage = g_drop_weight_stage;
+        a.fuse = x.fuse_act ? 1 : 0;
+        a.act_out = x.fuse_act ? *x.fuse_act : SplOperand{nullptr, nullptr, RN, 1};
+        a.in_squares = x.in_squares; a.in_groups = x.in_dim / 64; a.in_dim = float(x.in_dim); a.eps = x.eps;
+        const SplOperand emit_out = x.emit_out ? *x.emit_out : SplOperand{nullptr, nullptr, RN, 1};
+        a.emit_weight = x.emit_weight; a.emit_out = emit_out; a.emit_squares = x.emit_squares;
+        const dim3 grid(cut.pieces * row_blocks), block(SPL_TC_THREADS);
         // The pair form, two tiles of the weight a block against one stream of activations.
         const int splits = pair_splits(w, scratch.sms, row_blocks, x.fuse_act != nullptr);
         if (splits > 0) {
@@ -379,8 +412,6 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
             }
             return true;
         }
-    }
-    if constexpr (RN == 128) {
         if (x.fuse_act) launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_FUSE>, grid, block, spl_tc_smem_bytes(RN), stream, a);
         else if (x.emit_weight && cut.splits == 1) launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_EMIT>, grid, block, spl_tc_smem_bytes(RN), stream, a);
         else launch_step(spl_gemm_q4_tc_kernel<RN, SPL_TC_PLAIN>, grid, block, spl_tc_smem_bytes(RN), stream, a);
@@ -394,8 +425,8 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
             launch_step(spl_gemm_fixup_kernel, dim3(blocks), dim3(256), 0, stream, (const float *)scratch.slots, cut.splits, cut.pieces, RN, rows, w.tiles, w.ld, w.interleave,
                         residual, out, x.emit_weight, emit_out, x.emit_squares);
         }
+        return true;
     }
-    return true;
 }
 
 // out[r][:] = GEMM(w, operand[r][:]) (+ residual) for the first `rows` rows of the operand. False when the scratch is too small.
@@ -468,7 +499,7 @@ void launch_gemm_gguf(cudaStream_t stream, const SplGgufDev &w, const GemmOperan
 bool launch_gemm(spl_engine *e, const SplQ4Dev &w, const GemmOperand &op, float *out, const float *residual, int rows, const GemmExtras &x = GemmExtras()) {
     profile_begin(e, KLASS_GEMM, double(w.bytes()) * ((rows + op.rn - 1) / op.rn));
     --e->launches;      // profile_begin counted one; the launcher counts the kernels it really starts
-    const GemmScratch scratch{e->slots, e->slot_floats, e->tc_error, e->sms, e};
+    const GemmScratch scratch{e->slots, e->slot_floats, e->tc_error, e->sms, e->clusters, e};
     const bool fits = launch_gemm_rows(e->stream, w, op, out, residual, rows, scratch, x, &e->launches);
     profile_end(e);
     return fits;
@@ -810,7 +841,7 @@ spl_status create(const spl_geometry *gp, const spl_config *cp, spl_engine *e) {
     if (prop.major != 10) return e->fail(SPL_ERR_UNSUPPORTED_DEVICE, "unsupported device: kernels are built for sm_100a only");
     e->device = cp->device;
     SPL_CUDA(cudaSetDevice(e->device));
-    if (!configure_device(e->device, &e->sms)) return e->fail(SPL_ERR_UNSUPPORTED_DEVICE, "unsupported device: the kernels' shared-memory opt-in failed");
+    if (!configure_device(e->device, &e->sms, &e->clusters)) return e->fail(SPL_ERR_UNSUPPORTED_DEVICE, "unsupported device: the kernels' shared-memory opt-in failed");
     spl_status hs = spl_host_create(gp, cp, &e->host);
     if (hs != SPL_OK) return e->fail(hs, "invalid engine configuration");
     e->c = e->host->config;
@@ -1444,6 +1475,16 @@ spl_status spl_debug_gguf_plan(int32_t format, int32_t n, int32_t k, int32_t row
     return SPL_OK;
 }
 
+spl_status spl_debug_q4_plan(int32_t n, int32_t k, int32_t sms, const int32_t *clusters, int32_t *pieces) {
+    if (n <= 0 || k <= 0 || k % 256 || sms <= 0 || !clusters || !pieces) return SPL_ERR_INVALID_ARGUMENT;
+    SplQ4Dev w;
+    w.n = n; w.ld = round16(n); w.tiles = (n + 127) / 128; w.k = k;
+    int resident[SPL_NARROW_CLUSTER + 1] = {};
+    for (int s = 1; s <= SPL_NARROW_CLUSTER; ++s) resident[s] = clusters[s - 1];
+    *pieces = narrow_splits(w, sms, resident, false);
+    return SPL_OK;
+}
+
 spl_status spl_debug_gguf_block_rows(spl_engine *e, int32_t rows) {
     if (!e || (rows != 0 && rows != 64 && rows != 128)) return SPL_ERR_INVALID_ARGUMENT;
     e->gguf_block_rows = rows;
@@ -1809,7 +1850,7 @@ extern "C" spl_status spl_gemm_q4_static(spl_engine *e, int32_t layer, int32_t w
     // that are never stored, and every slot the second kernel reads is written by this call.
     SPL_CUDA(cudaMemsetAsync(control, 0, SPL_STATIC_CONTROL_BYTES, stream));
     spl_operand_kernel<<<rows, 256, 0, stream>>>(device_activations, SplOperand{operand, sums, rn, 1}, w->k);
-    const GemmScratch scratch{slots, SPL_STATIC_SLOT_BYTES / 4, control, e->sms};
+    const GemmScratch scratch{slots, SPL_STATIC_SLOT_BYTES / 4, control, e->sms, e->clusters};
     if (!launch_gemm_rows(stream, *w, GemmOperand{operand, sums, rn, 1}, device_out, device_residual, rows, scratch, GemmExtras(), nullptr))
         return e->fail(SPL_ERR_INVALID_ARGUMENT, "spl_gemm_q4_static: the tensor does not fit the static scratch");
     return check_launch(e, "spl_gemm_q4_static");
@@ -1840,7 +1881,7 @@ spl_status spl_op_gemm_q4(int32_t device, const uint32_t *packed, const uint16_t
     spl_engine *e = &local;
     e->device = device;
     SPL_CUDA(cudaSetDevice(device));
-    if (!configure_device(device, &e->sms)) return SPL_ERR_UNSUPPORTED_DEVICE;
+    if (!configure_device(device, &e->sms, &e->clusters)) return SPL_ERR_UNSUPPORTED_DEVICE;
     SPL_CUDA(cudaStreamCreate(&e->stream));
     SplQ4Dev w;
     spl_status s = alloc_q4(e, w, n, k);
@@ -1862,7 +1903,7 @@ spl_status spl_op_gemm_q4(int32_t device, const uint32_t *packed, const uint16_t
         cudaMemcpyAsync(d_act32, activations, size_t(rows) * k * 4, cudaMemcpyHostToDevice, e->stream);
         spl_operand_kernel<<<rows, 256, 0, e->stream>>>(d_act32, SplOperand{d_act, d_sums, rn, blocks}, k);
         if (residual) cudaMemcpy2DAsync(d_out, size_t(ld) * 4, residual, size_t(n) * 4, size_t(n) * 4, rows, cudaMemcpyHostToDevice, e->stream);
-        const GemmScratch scratch{e->slots, e->slot_floats, d_flag, e->sms};
+        const GemmScratch scratch{e->slots, e->slot_floats, d_flag, e->sms, e->clusters};
         if (!launch_gemm_rows(e->stream, w, GemmOperand{d_act, d_sums, rn, blocks}, d_out, residual ? d_out : nullptr, rows, scratch, GemmExtras(), nullptr)) s = SPL_ERR_INVALID_ARGUMENT;
         if (s == SPL_OK) s = check_launch(e, "gemm");
         if (cudaStreamSynchronize(e->stream) != cudaSuccess) s = SPL_ERR_DEVICE;
@@ -1889,7 +1930,7 @@ spl_status spl_op_gemm_gguf(int32_t device, int32_t format, const uint8_t *block
     spl_engine *e = &local;
     e->device = device;
     SPL_CUDA(cudaSetDevice(device));
-    if (!configure_device(device, &e->sms)) return SPL_ERR_UNSUPPORTED_DEVICE;
+    if (!configure_device(device, &e->sms, &e->clusters)) return SPL_ERR_UNSUPPORTED_DEVICE;
     SPL_CUDA(cudaStreamCreate(&e->stream));
     SplGgufDev w;
     w.n = n; w.ld = round16(n); w.tiles = (n + 127) / 128; w.k = k; w.format = format;
@@ -2023,7 +2064,7 @@ static spl_status pass_gemm(spl_engine *e, const SplQ4Dev &w, const float *devic
     const int rn = operand_rn(rows), blocks = (rows + rn - 1) / rn;
     const SplOperand operand{e->act, e->act_sums, rn, blocks};
     launch_step(spl_operand_kernel, dim3(rows), dim3(256), 0, e->stream, device_in, operand, w.k);
-    const GemmScratch scratch{e->slots, e->slot_floats, e->tc_error, e->sms};
+    const GemmScratch scratch{e->slots, e->slot_floats, e->tc_error, e->sms, e->clusters};
     if (!launch_gemm_rows(e->stream, w, GemmOperand{e->act, e->act_sums, rn, blocks}, device_out, device_residual, rows, scratch, GemmExtras(), nullptr))
         return e->fail(SPL_ERR_INVALID_ROWS, "invalid step rows: the GEMM scratch is smaller than the call needs");
     return check_launch(e, "spl_pass_gemm");

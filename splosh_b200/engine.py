@@ -212,6 +212,7 @@ def lib():
             "spl_debug_kv_store": (i32, [vp, i32]),
             "spl_debug_gdn_chunk_min": (i32, [vp, i32]),
             "spl_debug_gguf_plan": (i32, [i32, i32, i32, i32, i32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
+            "spl_debug_q4_plan": (i32, [i32, i32, i32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
             "spl_debug_gguf_block_rows": (i32, [vp, i32]),
             "spl_debug_pair_blocks": (i32, [vp, i32]),
             "spl_debug_wait_budget": (i32, [vp, C.c_int64]),
@@ -747,6 +748,15 @@ RESIDENT = ["in_proj", "out_proj", "gate_up", "down", "head"]
 def debug_pair_blocks(enabled=True):
     """Steps of more than 64 rows on the pair form of the 128-row GEMM block (default) or on the one-tile block (process-wide)."""
     lib().spl_debug_pair_blocks(None, int(enabled))
+
+
+def debug_q4_plan(n, k, sms=148, clusters=(148, 74, 45, 33, 26, 22, 15, 15)):
+    """Pieces of the contraction of an MLX affine-4 GEMM of up to 64 rows (`clusters`: how many clusters of 1 ... 8 blocks are resident); no device needed."""
+    pieces = C.c_int32(0)
+    status = lib().spl_debug_q4_plan(n, k, sms, (C.c_int32 * 8)(*clusters), C.byref(pieces))
+    if status:
+        raise EngineError(status, "spl_debug_q4_plan refused its arguments")
+    return pieces.value
 
 
 def debug_gguf_plan(kind, n, k, rows, sms=148):

@@ -67,6 +67,15 @@ def test_row_edges_over_one_and_several_tiles_a_block_and_cut_tiles(oracle, n, k
     case(oracle, n, k, rows, n + k + rows, residual=rows % 2 == 0)
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("n,k,pieces", [(128, 4096, 8), (128, 3840, 8), (1024, 5120, 7), (2048, 5120, 5), (19216, 2560, 1)])
+def test_row_edges_over_the_largest_clusters_and_long_tiles(oracle, n, k, pieces, rows):
+    """Clusters of eight blocks of whole and of unequal length (15 stages: the last block has one of two), of seven and of five, and a tensor of 151 uncut
+    tiles of ten stages: the blocks that take a second tile go round every ring across the boundary. TOL is the order of the sums, as above."""
+    assert S.engine.debug_q4_plan(n, k) == pieces
+    case(oracle, n, k, rows, n + k + rows, residual=rows % 2 == 0)
+
+
 @pytest.mark.parametrize("n,k", [(17408, 5120), (5120, 17408), (10240, 5120), (5120, 6144)])
 def test_27b_shapes_at_64_rows(oracle, n, k):
     case(oracle, n, k, 64, 7)
