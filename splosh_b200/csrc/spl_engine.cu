@@ -354,6 +354,7 @@ template <int RN>
 bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &op, float *out, const float *residual, int rows,
                     const GemmScratch &scratch, const GemmExtras &x, int *launches) {
     if constexpr (RN < 128) {
+        if (rows > RN || op.blocks != 1) return false;          // one row block: the kernel knows no other
         // The narrow block: a cut tile's pieces are a cluster of blocks, one tile a cluster; a block of an uncut tensor stays and takes every gridDim.x-th tile.
         const int splits = narrow_splits(w, scratch.sms, scratch.clusters, x.fuse_act != nullptr);
         SplNarrowArgs n = {};
