@@ -460,10 +460,11 @@ spl_status spl_draft_debug_read(spl_draft *draft, int32_t what, int32_t index, v
  * path because cudaMalloc and cudaFree synchronise the whole device.
  * This entry point runs out[r][:] = GEMM(weights, activations[r][:]) (+ residual) on one of the
  * engine's resident weights and calls no cudaMalloc, cudaFree or other allocating routine: the
- * GEMM operand, its per-64 sums, the partial sums of a cut contraction and the calls' error words live in a
- * static device array of about 12.3 MiB that every GPU loading the library holds until exit.
+ * GEMM operand, its per-64 sums and the calls' error words live in a
+ * static device array of about 2.3 MiB that every GPU loading the library holds until exit.
  *   - all three buffers are DEVICE pointers: activations fp32 [rows][inner], residual (may be
- *     null, may alias out) and out fp32 [rows][ld], ld = the tensor's columns rounded up to 16;
+ *     null, may alias out) and out fp32 [rows][ld], ld = the tensor's columns rounded up to 16; residual
+ *     and out may begin at any float;
  *   - rows must be 1..64 and the tensor's inner dimension at most 17408, else SPL_ERR_INVALID_ROWS
  *     / SPL_ERR_INVALID_ARGUMENT with the reason in spl_last_error_string;
  *   - the first call on a device looks up the array's address (cudaGetSymbolAddress); make that

@@ -1766,17 +1766,14 @@ spl_status spl_kv_import(spl_engine *e, int32_t slot, int32_t token_count, const
 // For callers that may not allocate device memory: a host that handed the whole GPU to its own
 // pool at start-up, or a serving loop that bans allocator calls on its hot path because
 // cudaMalloc and cudaFree synchronise the whole device. The scratch the ordinary path takes from the engine's buffers (the bf16 operand with its
-// per-64 sums, and the slots where the blocks of a cut tile leave their partial sums) lives here in
-// one file-scope device array, so every GPU that loads the library holds SPL_STATIC_BYTES (about 12.3 MiB) until the
-// process exits.
+// per-64 sums; the blocks of a cut tile meet in a cluster and leave nothing) lives here in one file-scope device array, so every GPU that loads the
+// library holds SPL_STATIC_BYTES (about 2.3 MiB) until the process exits.
 #define SPL_STATIC_ROWS 64
 #define SPL_STATIC_INNER 17408
 #define SPL_STATIC_OPERAND_BYTES (SPL_STATIC_ROWS * SPL_STATIC_INNER * 2)
 #define SPL_STATIC_SUMS_BYTES (SPL_STATIC_ROWS * ((SPL_STATIC_INNER / 64 + 15) / 16) * 128)      // tiles of split means
 #define SPL_STATIC_CONTROL_BYTES 256       // the error words
-#define SPL_STATIC_SLOTS 320               // room for partial sums, in units of 64 x 128 floats: splits x 64 rows x the tensor's columns must fit (else the call is refused)
-#define SPL_STATIC_SLOT_BYTES (SPL_STATIC_SLOTS * 64 * 128 * 4)
-#define SPL_STATIC_BYTES (SPL_STATIC_OPERAND_BYTES + SPL_STATIC_SUMS_BYTES + SPL_STATIC_CONTROL_BYTES + SPL_STATIC_SLOT_BYTES)
+#define SPL_STATIC_BYTES (SPL_STATIC_OPERAND_BYTES + SPL_STATIC_SUMS_BYTES + SPL_STATIC_CONTROL_BYTES)
 static __device__ __align__(256) unsigned char spl_static_scratch[SPL_STATIC_BYTES];
 // The array's address on each device, asked for once per device. The symbol itself is only a
 // host-side handle: a kernel must be given what cudaGetSymbolAddress returns.
@@ -1843,17 +1840,16 @@ extern "C" spl_status spl_gemm_q4_static(spl_engine *e, int32_t layer, int32_t w
     __nv_bfloat16 *operand = reinterpret_cast<__nv_bfloat16 *>(base);
     float *sums = reinterpret_cast<float *>(base + SPL_STATIC_OPERAND_BYTES);
     int *control = reinterpret_cast<int *>(base + SPL_STATIC_OPERAND_BYTES + SPL_STATIC_SUMS_BYTES);
-    float *slots = reinterpret_cast<float *>(base + SPL_STATIC_OPERAND_BYTES + SPL_STATIC_SUMS_BYTES + SPL_STATIC_CONTROL_BYTES);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
     const int rn = operand_rn(rows);
     // The array keeps what the last call left. The error words have to start at zero; the
-    // operand and sums of the rows in use are rewritten here, the block's other rows feed outputs
-    // that are never stored, and every slot the second kernel reads is written by this call.
+    // operand and sums of the rows in use are rewritten here, and the block's other rows feed outputs
+    // that are never stored.
     SPL_CUDA(cudaMemsetAsync(control, 0, SPL_STATIC_CONTROL_BYTES, stream));
     spl_operand_kernel<<<rows, 256, 0, stream>>>(device_activations, SplOperand{operand, sums, rn, 1}, w->k);
-    const GemmScratch scratch{slots, SPL_STATIC_SLOT_BYTES / 4, control, e->sms, e->clusters};
+    const GemmScratch scratch{nullptr, 0, control, e->sms, e->clusters};
     if (!launch_gemm_rows(stream, *w, GemmOperand{operand, sums, rn, 1}, device_out, device_residual, rows, scratch, GemmExtras(), nullptr))
-        return e->fail(SPL_ERR_INVALID_ARGUMENT, "spl_gemm_q4_static: the tensor does not fit the static scratch");
+        return e->fail(SPL_ERR_INVALID_ARGUMENT, "spl_gemm_q4_static: more rows than the GEMM's block holds");
     return check_launch(e, "spl_gemm_q4_static");
 }
 
