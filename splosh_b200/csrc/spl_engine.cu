@@ -287,13 +287,13 @@ static int g_pair_blocks = 1;
 // `whole`: the block's output stage needs the whole sum (the fused SiLU gate), so tiles are not cut.
 struct GemmCut { int pieces, splits; };
 GemmCut gemm_cut(const SplQ4Dev &w, int sms, int row_blocks, bool whole) {
-    const int stages = w.k / (64 * spl_tc_super(128));
+    const int stages = w.k / (64 * SPL_TC_WIDE_SUPER);
     int best = 1; double best_cost = 1e30;
     for (int s = 1; s <= stages && s <= 16 && !(whole && s > 1); ++s) {
         const int per = (stages + s - 1) / s;
         if (s > 1 && per < 2) break;
         const int waves = (w.tiles * s * row_blocks + sms - 1) / sms;
-        const double cost = double(waves) * (per * spl_tc_super(128) + 20.0) + (s > 1 ? 12.0 : 0.0);      // in groups of time: a block's fill and output cost about twenty, the second kernel twelve
+        const double cost = double(waves) * (per * SPL_TC_WIDE_SUPER + 20.0) + (s > 1 ? 12.0 : 0.0);      // in groups of time: a block's fill and output cost about twenty, the second kernel twelve
         if (cost < best_cost - 1e-9) { best_cost = cost; best = s; }
     }
     return {w.tiles * best, best};
@@ -384,7 +384,7 @@ bool launch_gemm_tc(cudaStream_t stream, const SplQ4Dev &w, const GemmOperand &o
         SplGemmArgs a = {};
         a.codes = w.codes; a.sb = w.sb; a.act = op.values; a.act_sums = op.sums; a.out = out; a.residual = residual;
         a.slots = scratch.slots; a.error_flag = scratch.error_flag;
-        a.out_ld = w.ld; a.rows = rows; a.op_blocks = op.blocks; a.tiles = w.tiles; a.stages_per_tile = w.k / (64 * spl_tc_super(RN)); a.interleave = w.interleave;
+        a.out_ld = w.ld; a.rows = rows; a.op_blocks = op.blocks; a.tiles = w.tiles; a.stages_per_tile = w.k / (64 * SPL_TC_WIDE_SUPER); a.interleave = w.interleave;
         a.pieces = cut.pieces; a.row_blocks = row_blocks; a.splits = cut.splits;
         a.drop_stage = g_drop_weight_stage;
         a.fuse = x.fuse_act ? 1 : 0;

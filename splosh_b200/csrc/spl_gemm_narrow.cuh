@@ -100,8 +100,8 @@ __device__ __forceinline__ void spl_narrow_output(const SplNarrowArgs &a, const 
         // elements. act = bf16(silu(gate) * up) (Sources/Shaders/engine.metal:200-219) into the next GEMM's operand, a warp a row.
         const int e = 2 * lane, gc = (e >> 4) * 32 + (e & 15);
 #pragma unroll 1
-        for (int k0 = 0; split * WARPS + warp + k0 * WARPS * S < a.rows; k0 += PRE) {
-            float2 g[PRE], u[PRE];          // (never of a cut tile)
+        for (int k0 = 0; warp + k0 * WARPS < a.rows; k0 += PRE) {          // (never of a cut tile)
+            float2 g[PRE], u[PRE];
 #pragma unroll
             for (int k = 0; k < PRE; ++k) {
                 const uint32_t at = base + uint32_t(min(warp + (k0 + k) * WARPS, RN - 1) * 128 + gc) * 4;
@@ -109,7 +109,7 @@ __device__ __forceinline__ void spl_narrow_output(const SplNarrowArgs &a, const 
             }
 #pragma unroll
             for (int k = 0; k < PRE; ++k) {
-                const int row = split * WARPS + warp + (k0 + k) * WARPS * S;
+                const int row = warp + (k0 + k) * WARPS;
                 const float v0 = spl_bf16_to_float(spl_float_to_bf16(spl_silu_exact(g[k].x) * u[k].x)), v1 = spl_bf16_to_float(spl_float_to_bf16(spl_silu_exact(g[k].y) * u[k].y));
                 // The sum in one fixed order: neighbours, then a butterfly over the rest.
                 float s = v0 + v1;

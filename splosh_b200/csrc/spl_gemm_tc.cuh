@@ -328,18 +328,14 @@ __device__ __forceinline__ void spl_set_barrier(int set) {
 #define SPL_TC_PAIR_CSTAGES 4
 #define SPL_TC_PAIR_AUNITS 3
 
-// The one-tile block of 128 rows (an instruction is 128 x 128 x 16): stages of two groups, so that four stages of activations still fit in shared
+// The one-tile block of 128 rows (an instruction is 128 x 128 x 16): stages of two groups, one unit, so that four stages of activations still fit in shared
 // memory, and one issuing warp with one accumulator: an instruction then keeps the tensor pipe 64 cycles and one warp issues at that rate.
-__host__ __device__ constexpr int spl_tc_super(int rn) { return rn >= 128 ? 2 : 4; }          // groups per stage (four: the narrow block, spl_gemm_narrow.cuh)
-__host__ __device__ constexpr int spl_tc_issuers(int) { return 1; }        // issuing warps = units per stage
-// Stages of activations: held until the tensor core has finished with them. Stages of codes with their scale/bias
-// words: handed back as soon as they are in registers.
-__host__ __device__ constexpr int spl_tc_bstages(int) { return 4; }
-__host__ __device__ constexpr int spl_tc_cstages(int) { return 4; }
-__host__ __device__ constexpr size_t spl_tc_bstage_bytes(int rn) { return size_t(spl_tc_super(rn)) * size_t(rn) * 128; }
+#define SPL_TC_WIDE_SUPER 2      // groups per stage
+#define SPL_TC_WIDE_BSTAGES 4    // stages of activations: held until the tensor core has finished with them
+#define SPL_TC_WIDE_CSTAGES 4    // stages of codes with their scale/bias words: handed back as soon as they are in registers
 #define SPL_TC_CONTROL_BYTES 4096       // barriers, row factors, the output stage's exchange cells
 __host__ __device__ constexpr size_t spl_tc_smem_bytes(int rn) {
-    return 1024 /* alignment slack */ + size_t(spl_tc_cstages(rn)) * spl_tc_super(rn) * (4096 + 512) + size_t(spl_tc_bstages(rn)) * spl_tc_bstage_bytes(rn)
+    return 1024 /* alignment slack */ + size_t(SPL_TC_WIDE_CSTAGES) * SPL_TC_WIDE_SUPER * (4096 + 512) + size_t(SPL_TC_WIDE_BSTAGES) * SPL_TC_WIDE_SUPER * rn * 128
            + size_t(2) * rn * 128 /* tiles of split means */ + SPL_TC_CONTROL_BYTES;
 }
 __host__ __device__ constexpr size_t spl_tc_pair_smem_bytes() {
@@ -401,7 +397,6 @@ __device__ __noinline__ bool spl_tc_output_stage(const SplGemmArgs &args, const 
     a.in_squares = args.in_squares;
     a.emit_weight = args.emit_weight; a.emit_squares = args.emit_squares;
     a.emit_out.values = args.emit_out.values; a.emit_out.sums = args.emit_out.sums; a.emit_out.rn = args.emit_out.rn; a.emit_out.blocks = args.emit_out.blocks;
-    constexpr int NW = spl_tc_issuers(RN);
     const uint32_t tmem_d = o.tmem_d, lane_base = o.lane_base;
     const int rb = o.rb, tile = o.tile, set = o.set, quarter = o.quarter, col = o.col, lane = o.lane;
     int *abort_word = o.abort_word;
@@ -422,12 +417,6 @@ __device__ __noinline__ bool spl_tc_output_stage(const SplGemmArgs &args, const 
             spl_tc_ld16(v0, tmem_d + lane_base + c0);
 #pragma unroll
             for (int r = 0; r < 16; ++r) total[r] = __uint_as_float(v0[r]);
-            if (NW == 2) {
-                uint32_t v1[16];
-                spl_tc_ld16(v1, tmem_d + lane_base + RN + c0);
-#pragma unroll
-                for (int r = 0; r < 16; ++r) total[r] += __uint_as_float(v1[r]);
-            }
         }
         // The rows' factors of a deferred norm: a cut tile's partial sums are scaled one by one, so their sum is.
         if (a.in_squares)
@@ -537,8 +526,8 @@ __device__ __noinline__ bool spl_tc_output_stage(const SplGemmArgs &args, const 
 template <int RN, int MODE>
 __global__ void __launch_bounds__(SPL_TC_THREADS, 1)
 spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
-    constexpr int BST = spl_tc_bstages(RN), CST = spl_tc_cstages(RN), AUN = SPL_TC_AUNITS, SUPER = spl_tc_super(RN), UPS = SUPER / 2, NW = spl_tc_issuers(RN);
-    static_assert(UPS == NW, "every issuing warp takes one unit of every stage");
+    constexpr int BST = SPL_TC_WIDE_BSTAGES, CST = SPL_TC_WIDE_CSTAGES, AUN = SPL_TC_AUNITS, SUPER = SPL_TC_WIDE_SUPER;
+    static_assert(SUPER == 2, "a stage is a unit");
     constexpr int BTILE = SUPER * RN * 128, WSTAGE = SUPER * 4096, QSTAGE = SUPER * 128, TTILE = RN * 128;
     extern __shared__ unsigned char spl_tc_smem_raw[];
     // The swizzled activation tiles must sit on 1,024-byte boundaries.
@@ -556,7 +545,7 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
     float *cells = row_factor + 128;                                                    // [SETS][4 warps][16 rows][2] the output stage's exchange
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int W_COPY = SPL_TC_SETS * 4, W_MMA0 = W_COPY + 1, W_COPYB = W_COPY + 2, W_MMA1 = W_COPY + 3;
+    constexpr int W_COPY = SPL_TC_SETS * 4, W_MMA0 = W_COPY + 1, W_COPYB = W_COPY + 2;         // the block's last warp has no role
     const int rb = int(blockIdx.x) % a.row_blocks, c = int(blockIdx.x) / a.row_blocks, row_blocks = a.op_blocks, S = a.stages_per_tile;
     // This block's piece: an equal share of the stages of its tile (the host keeps splits <= S, so no piece is empty).
     // Stages are counted along the weight array: stage w is stage w % S of tile w / S.
@@ -592,12 +581,11 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
         const int total = int(finished + 1 - bars);
         for (int b = lane + CST; b < total; b += 32) {
             uint64_t *bar = bars + b;
-            const uint32_t count = bar < full_b ? uint32_t(4 * UPS)   // empty_c: the sets (four warps each) that take the stage's units
+            const uint32_t count = bar < full_b ? 4u              // empty_c: the set (four warps) that takes the stage's unit
                                  : bar < done ? 1u                // full_b: the copy's bytes
-                                 : bar < full_a ? 1u              // done: the commit of the issuing warp that took the unit
+                                 : bar < full_a ? 1u              // done: the commit behind the unit's instructions
                                  : bar < full_t ? 4u              // full_a (one per unit modulo 2 AUN): the four warps of a set
-                                 : bar < empty_t ? 1u             // full_t
-                                 : uint32_t(NW);                  // empty_t and finished: the issuing warps
+                                 : 1u;                            // full_t; empty_t and finished: the issuing warp's commits
             spl_mbar_init(bar, count);
         }
         if (lane == 0) *abort_word = 0;
@@ -611,8 +599,7 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
     __syncthreads();
     spl_tc_fence_after();
     const uint32_t tmem = *tmem_slot;                 // lane 0, first allocated column
-    // The accumulators, one per issuing warp (instructions of different warps are not ordered against each other), in
-    // columns [0, 128); the A ring, 64 columns a unit; the second-term operand, 8 columns a unit.
+    // The accumulator in columns [0, 128); the A ring, 64 columns a unit; the second-term operand, 8 columns a unit.
     const uint32_t tmem_d = tmem, tmem_a = tmem + 128, tmem_aq = tmem + 128 + AUN * 64;
     bool ok = true;
     spl_grid_begin();
@@ -646,10 +633,8 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
                     spl_bulk_g2s(t_ring + slot * TTILE, tsrc + (size_t(want) * row_blocks + rb) * TTILE, TTILE, &full_t[slot]);
                     mean_tile = want; ++mean_loads; issued_t = mean_loads;
                 }
-                if (i >= BST) {            // the stage's last tenant: its units have to have completed
-                    bool freed = true;
-                    for (int h = 0; h < UPS; ++h) { const int u = UPS * (i - BST) + h; freed = freed && spl_mbar_wait(&done[u & 15], (u >> 4) & 1, abort); }
-                    if (!freed) { ok = false; if (!*abort) spl_note_wait(a.error_flag, 21, i); break; }
+                if (i >= BST && !spl_mbar_wait(&done[(i - BST) & 15], ((i - BST) >> 4) & 1, abort)) {            // the stage's last tenant has to have completed
+                    ok = false; if (!*abort) spl_note_wait(a.error_flag, 21, i); break;
                 }
                 issued_b = i + 1;
                 spl_mbar_expect_tx(&full_b[sbq], BTILE);
@@ -663,65 +648,54 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
                 }
             }
         }
-    } else if (warp == W_MMA0 || warp == W_MMA1) {
+    } else if (warp == W_MMA0) {
         // ---- tensor-core issue: D[128 x RN] += A[128 x 64] (fp16, tensor memory) * B[RN x 64]^T (fp16, shared memory).
-        // The whole warp runs the loop and its waits; one elected lane issues (spl_elect_one). An elected lane is held
-        // while the tensor pipe works through its instructions, and a wait on a barrier costs its latency even when the
-        // phase is complete, so in the narrow blocks two warps take the units in turn (one the first unit of every stage,
-        // the other the second), each into an accumulator of its own: one warp's waits run under the other's
-        // instructions. A unit is eight k16 instructions at fixed offsets from the unit's bases and a ninth for its share
-        // of the second term (the unit's 8 values of that contraction; the other 8 columns of its operand slot are zero).
-        const int m = warp == W_MMA0 ? 0 : 1;
-        if (m < NW) {
+        // The whole warp runs the loop and its waits; one elected lane issues (spl_elect_one). A unit is eight k16 instructions at fixed
+        // offsets from the unit's bases and a ninth for its share of the second term (the unit's 8 values of that contraction; the
+        // other 8 columns of its operand slot are zero).
         constexpr uint32_t idesc = spl_tc_idesc(RN);
         int mean_tile = -1, mean_loads = 0, mean_slot = 0;
         const uint64_t b_desc0 = spl_tc_desc_sw128(spl_smem_addr(b_ring)), t_desc0 = spl_tc_desc_sw128(spl_smem_addr(t_ring));
-        const uint32_t d_mine = tmem_d + m * RN;
-        // A unit's operand slot is un % AUN, but its "converted" barrier is un % (2 AUN): the slots alternate between the two
-        // issuing warps (AUN is odd), so with one barrier a slot a warp that runs ahead of the other would meet the barrier
-        // two uses behind and take the previous tenant's completion for its own unit's. Barrier un % (2 AUN) belongs to one warp.
-        int slot = m, fa = m;                              // un % AUN, un % (2 AUN)
-        uint32_t a_parity = 0;                             // (un / (2 AUN)) & 1
+        int slot = 0, fa = 0;                              // i % AUN (the operand slot), i % (2 AUN) (its "converted" barrier)
+        uint32_t a_parity = 0;                             // (i / (2 AUN)) & 1
         for (int i = 0; i < stages; ++i) {
-            const int un = UPS * i + m, j = (w0 + place(i)) % S, sbq = i % BST;
-            const int gu = j * UPS + m;                    // the unit's place in the contraction: 8 units to a tile of means, 2 to a k16 of the second term
+            const int j = (w0 + place(i)) % S, sbq = i % BST;       // j, the unit's place in the contraction: 8 units to a tile of means, 2 to a k16 of the second term
             const bool first = i == 0, last = i + 1 == stages;
-            const uint64_t b_desc = b_desc0 + uint64_t((sbq * BTILE + m * 2 * RN * 128) >> 4);
+            const uint64_t b_desc = b_desc0 + uint64_t((sbq * BTILE) >> 4);
             const uint32_t a_base = tmem_a + slot * 64;
-            const int want = gu >> 3;
+            const int want = j >> 3;
             if (want != mean_tile) {
                 if (mean_tile >= 0 && spl_elect_one()) spl_tc_commit(&empty_t[mean_slot]);      // every instruction of this warp that read the old tile has been issued
                 __syncwarp();
                 mean_slot = mean_loads & 1;
-                if (!spl_mbar_wait_warp(&full_t[mean_slot], (mean_loads >> 1) & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 30 + m, i); break; }
+                if (!spl_mbar_wait_warp(&full_t[mean_slot], (mean_loads >> 1) & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 30, i); break; }
                 mean_tile = want; ++mean_loads;
             }
-            if (!spl_mbar_wait_warp(&full_b[sbq], (i / BST) & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 34 + m, i); break; }
-            if (!spl_mbar_wait_warp(&full_a[fa], a_parity, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 36 + m, i); break; }
+            if (!spl_mbar_wait_warp(&full_b[sbq], (i / BST) & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 34, i); break; }
+            if (!spl_mbar_wait_warp(&full_a[fa], a_parity, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 36, i); break; }
             spl_tc_fence_after();
-            const uint64_t t_desc = t_desc0 + uint64_t((mean_slot * TTILE + ((gu >> 1) & 3) * 32) >> 4);
+            const uint64_t t_desc = t_desc0 + uint64_t((mean_slot * TTILE + ((j >> 1) & 3) * 32) >> 4);
             if (!first) {                                        // the common case: nothing to decide between the instructions
                 if (spl_elect_one()) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
-                        spl_tc_mma_ts_acc(d_mine, a_base + q * 8, b_desc + uint64_t(((q >> 2) * RN * 128 + (q & 3) * 32) >> 4), idesc);
-                    spl_tc_mma_ts_acc(d_mine, tmem_aq + slot * 8, t_desc, idesc);
-                    spl_tc_commit(&done[un & 15]);            // the unit's A slot is free, and with the stage's other unit its activations
+                        spl_tc_mma_ts_acc(tmem_d, a_base + q * 8, b_desc + uint64_t(((q >> 2) * RN * 128 + (q & 3) * 32) >> 4), idesc);
+                    spl_tc_mma_ts_acc(tmem_d, tmem_aq + slot * 8, t_desc, idesc);
+                    spl_tc_commit(&done[i & 15]);            // the unit's A slot is free, and its activations
                     if (last) spl_tc_commit(finished);
                 }
-            } else if (spl_elect_one()) {                        // the first unit of this warp overwrites its accumulator
+            } else if (spl_elect_one()) {                        // the first unit overwrites the accumulator
                 for (int q = 0; q < 8; ++q)
-                    spl_tc_mma_ts(d_mine, a_base + q * 8, b_desc + uint64_t(((q >> 2) * RN * 128 + (q & 3) * 32) >> 4), idesc, q ? 1u : 0u);
-                spl_tc_mma_ts_acc(d_mine, tmem_aq + slot * 8, t_desc, idesc);
-                spl_tc_commit(&done[un & 15]);
+                    spl_tc_mma_ts(tmem_d, a_base + q * 8, b_desc + uint64_t(((q >> 2) * RN * 128 + (q & 3) * 32) >> 4), idesc, q ? 1u : 0u);
+                spl_tc_mma_ts_acc(tmem_d, tmem_aq + slot * 8, t_desc, idesc);
+                spl_tc_commit(&done[i & 15]);
                 if (last) spl_tc_commit(finished);
             }
             __syncwarp();
-            slot += UPS; if (slot >= AUN) slot -= AUN;
-            fa += UPS; if (fa >= 2 * AUN) { fa -= 2 * AUN; a_parity ^= 1u; }
+            if (++slot == AUN) slot = 0;
+            if (++fa == 2 * AUN) { fa = 0; a_parity ^= 1u; }
         }
-        }
-    } else {
+    } else if (warp < W_COPY) {
         // ---- dequant: thread = output column; codes -> scale * (code - 8), exact in fp16 -> tensor memory. The sets
         // of four warps take the units of two groups in turn; a set's warps write the lanes of their
         // warp index mod 4. A unit also carries its two groups' pairs of the second-term operand.
@@ -755,21 +729,19 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
         out.abort_word = abort_word; out.row_factor = row_factor; out.cells = cells;
         // The conversion loop of the units that are this set's, then the output stage. j is the stage's place in its tile's contraction.
         {
-            const int un_end = UPS * stages;
 #pragma unroll 1
-            for (int un = set; ok && un < un_end; un += SPL_TC_SETS) {
-            const int i = un / UPS, h = un % UPS, sc = i % CST;
-            const int j = w0 + place(i) - tile * S;
-            if (!spl_mbar_wait_warp(&full_c[sc], (i / CST) & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 41, un); break; }
+            for (int un = set; ok && un < stages; un += SPL_TC_SETS) {
+            const int sc = un % CST;
+            const int j = w0 + place(un) - tile * S;
+            if (!spl_mbar_wait_warp(&full_c[sc], (un / CST) & 1, abort)) { ok = false; if (!*abort && lane == 0) spl_note_wait(a.error_flag, 41, un); break; }
             // The unit's codes and scale/bias words are read before anything is converted, so the codes can be handed back at once.
             uint4 lo[2], hi[2];
             uint32_t sbw[2];
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
-                const int u = 2 * h + v;
-                lo[v] = *reinterpret_cast<const uint4 *>(w_ring + size_t(sc) * WSTAGE + u * 4096 + col * 16);
-                hi[v] = *reinterpret_cast<const uint4 *>(w_ring + size_t(sc) * WSTAGE + u * 4096 + 2048 + col * 16);
-                sbw[v] = q_ring[sc * QSTAGE + u * 128 + col];
+                lo[v] = *reinterpret_cast<const uint4 *>(w_ring + size_t(sc) * WSTAGE + v * 4096 + col * 16);
+                hi[v] = *reinterpret_cast<const uint4 *>(w_ring + size_t(sc) * WSTAGE + v * 4096 + 2048 + col * 16);
+                sbw[v] = q_ring[sc * QSTAGE + v * 128 + col];
             }
             __syncwarp();
             if (lane == 0) spl_mbar_arrive(&empty_c[sc]);
@@ -792,7 +764,7 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {
                     const uint4 src = part == 0 ? lo[v] : hi[v];
-                        const uint32_t w4[4] = {src.x, src.y, src.z, src.w};
+                    const uint32_t w4[4] = {src.x, src.y, src.z, src.w};
                     uint32_t regs[16];
 #pragma unroll
                     for (int w = 0; w < 4; ++w)
@@ -811,7 +783,7 @@ spl_gemm_q4_tc_kernel(const __grid_constant__ SplGemmArgs a) {
             }
             // The unit's share of the second-term operand sits at its place among the sixteen values of its k16 instruction
             // (two units to an instruction, by the unit's place in the contraction); the rest is zero.
-            if (((j * UPS + h) & 1) == 0) { spl_tc_st4(tmem_aq + lane_base + slot * 8, aq[0], aq[1], aq[2], aq[3]); spl_tc_st4(tmem_aq + lane_base + slot * 8 + 4, 0u, 0u, 0u, 0u); }
+            if ((j & 1) == 0) { spl_tc_st4(tmem_aq + lane_base + slot * 8, aq[0], aq[1], aq[2], aq[3]); spl_tc_st4(tmem_aq + lane_base + slot * 8 + 4, 0u, 0u, 0u, 0u); }
             else { spl_tc_st4(tmem_aq + lane_base + slot * 8, 0u, 0u, 0u, 0u); spl_tc_st4(tmem_aq + lane_base + slot * 8 + 4, aq[0], aq[1], aq[2], aq[3]); }
             spl_tc_st_wait();
             spl_tc_fence_before();
@@ -1201,7 +1173,7 @@ spl_gemm_q4_pair_kernel(const uint32_t *__restrict__ codes, const uint32_t *__re
             for (int cb = set; cb < RN / 16; cb += SPL_TC_SETS) {
                 const int c0 = cb * 16;
                 float total[16];
-uint32_t v[16];
+                uint32_t v[16];
                 spl_tc_ld16(v, tmem_d + lane_base + om * RN + c0);
 #pragma unroll
                 for (int r = 0; r < 16; ++r) total[r] = __uint_as_float(v[r]);
