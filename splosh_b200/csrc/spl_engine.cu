@@ -266,7 +266,8 @@ bool configure_device(int device, int *sms, const int **clusters) {
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr; cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&resident[device][s], spl_gemm_q4_narrow_kernel<64>, &cfg) != cudaSuccess) return false;
+            // A size the device cannot hold is not used.
+            if (cudaOccupancyMaxActiveClusters(&resident[device][s], spl_gemm_q4_narrow_kernel<64>, &cfg) != cudaSuccess) { resident[device][s] = 0; cudaGetLastError(); }
         }
         if (cudaGetLastError() != cudaSuccess) return false;
         done[device] = true;
