@@ -382,7 +382,8 @@ spl_status spl_tensor_create_q4(spl_engine *engine, int32_t rows, int32_t inner,
 spl_status spl_tensor_create_vector(spl_engine *engine, const uint16_t *bf16, int32_t count, spl_tensor **out);
 void spl_tensor_destroy(spl_engine *engine, spl_tensor *tensor);
 spl_status spl_pass_begin(spl_engine *engine);
-/* Engine.gemm: out[r][:] = w x in[r][:] (+ residual[r][:]); in [rows][inner], out and residual [rows][w rows]. */
+/* Engine.gemm: out[r][:] = w x in[r][:] (+ residual[r][:]); in [rows][inner], out and residual [rows][w rows]. `in` begins on a 16-byte boundary;
+ * out and residual at any float up to 64 rows, on an 8-byte boundary above. */
 spl_status spl_pass_gemm(spl_engine *engine, const spl_tensor *weight, const float *device_in, int32_t rows, const float *device_residual, float *device_out);
 /* The target's lm_head: in [rows][hidden] -> out [rows][vocab]. */
 spl_status spl_pass_gemm_head(spl_engine *engine, const float *device_in, int32_t rows, float *device_out);

@@ -15,8 +15,9 @@
 //     gate's rows are taken several at a time, everything they need asked for first, and what the other outputs need is asked for before the sums are there.
 // The blocks of a cut tile are a cluster: the cluster's warps add the blocks' sums through distributed shared memory and write the output, with the
 // residual and the next deferred norm's operand. (They used to leave partial sums in global memory for a second kernel.)
-// Measured before and after, with those second kernels: gate|up (34,816 x 5,120) at 16 rows 34.8 -> 28 us, out and down together 16.5 -> 13.5 us a launch; a
-// step of the 27B shape with one row 6,617 -> 5,568 us, twelve rows 7,745 -> 6,706, 64 rows 10,979 -> 10,561.
+// Measured before and after, with those second kernels and the kernel that forms the operand: 5,120 x 6,144 at one row 13.5 -> 11.0 us, at 64 rows 16.6 -> 14.2;
+// 34,816 x 5,120 36.8 -> 28.4 and 40.0 -> 35.5; 1,024 x 5,120 9.2 -> 8.0 and 11.0 -> 10.4. A step of the 27B shape with one row 6,590 -> 5,489 us, twelve rows
+// 7,739 -> 6,584, 64 rows 11,191 -> 10,736.
 #pragma once
 #include "spl_gemm_tc.cuh"
 

@@ -8,22 +8,24 @@
 //
 // with a the bf16-rounded activations and sum(a) the fp32 per-64 sums of the rounded values.
 //
+// Here are the blocks of 128 rows (steps of more than 64) and what every q4 GEMM shares; the kernel of up to 64 rows is in spl_gemm_narrow.cuh.
+//
 // Shape of the computation. The product is taken transposed, D[n][r] = w[n][k] * a[r][k]^T, so
-// that 128 output columns are the M dimension of one tcgen05.mma and the step's rows (16..64 per
-// tile) are its N dimension. Per quant group (K = 64, four k16 instructions):
-//   * TMA bulk copies bring four groups at a time into shared memory, from two warps that run independently: one
-//     copies the weights (16 KiB of codes and 2 KiB of scale/bias words, a ring handed back as soon as the codes are
+// that 128 output columns are the M dimension of one tcgen05.mma and the rows (16, 32, 64 or 128 a
+// block) are its N dimension. Per quant group (K = 64, four k16 instructions):
+//   * TMA bulk copies bring two groups at a time into shared memory (the narrow kernel: four), from two warps that run independently: one
+//     copies the weights (of two groups 8 KiB of codes and 1 KiB of scale/bias words, a ring handed back as soon as the codes are
 //     in registers), the other the activations' slice (held until the tensor core has finished with it) and the
-//     tiles of split means, each of which serves sixteen groups;
+//     tiles of split means, each of which serves sixteen groups (the narrow kernel: with the stage);
 //   * dequant warps (one thread per output column, four sets of four warps taking units of two groups in turn)
 //     turn the codes into exact fp16 values scale * (code - 8), sixteen registers at a time, and write them into
 //     tensor memory as the A operand (tcgen05.st): weights never pass through shared memory expanded and are
 //     never re-read. A pair of weights costs one shift, one logic operation and one fused multiply-add;
 //   * the activations' producer already wrote them (bf16-rounded, held as fp16) in the
 //     128-byte-swizzled K-major image the tensor core reads as the B operand;
-//   * two warps issue the tcgen05.mma, a unit each in turn (eight k16 instructions and a ninth for the unit's
-//     share of the bias term), into an accumulator each; the accumulators stay in tensor memory for the whole
-//     contraction. The warps run their loops and waits whole, with one elected lane issuing;
+//   * tcgen05.mma is issued a unit at a time (eight k16 instructions and a ninth for the unit's share of the bias
+//     term), by one warp, or by two into an accumulator each (the pair form: a tile of the weight each; the narrow kernel: the
+//     units in turn); the accumulators stay in tensor memory for the whole contraction. The warps run their loops and waits whole, with one elected lane issuing;
 //   * the bias term, (bias + 8 scale) * sum(a) per group, comes from exact fp16 pairs of (64 bias, 512 scale)
 //     in tensor memory and the group means split in two fp16 numbers;
 //   * at the end every dequant warp reads its share of the accumulators (tcgen05.ld) and writes the output.
@@ -55,9 +57,10 @@ struct SplQ4Dev {
 // both operands in one 16-bit format, and the weights need fp16's 11 bits). A bf16 value of magnitude
 // 2^-14 .. 65504 is exact in fp16; a smaller one moves by at most 2^-25, below the fp32 accumulator's own
 // rounding for activations of order one. The per-64 sums are taken from the bf16 values themselves.
-// The operand is cut in 64-wide groups and in row blocks of RN rows (RN = 16, 32 or 64, fixed per step). Block (g, rb) is RN * 128 bytes: row r at (r / 8) * 1024 + (r % 8) * 128,
+// The operand is cut in 64-wide groups and in row blocks of RN rows (RN = 16, 32, 64 or 128, fixed per step). Block (g, rb) is RN * 128 bytes: row r at (r / 8) * 1024 + (r % 8) * 128,
 // its eight 16-byte units XOR-swizzled by r % 8: the canonical K-major SWIZZLE_128B image. The
-// per-64 sums sit beside it as tiles of the same shape, sixteen groups to a tile (SplOperand::put_sum).
+// per-64 sums sit beside it: in blocks of 128 rows as tiles of the same shape, sixteen groups to a tile; in smaller ones sixteen bytes
+// a row and pair of groups, plain, so that they travel with a stage of the activations (SplOperand::put_sum).
 // Four bf16-rounded values (as floats) -> four fp16 in two words.
 __device__ __forceinline__ uint2 spl_operand_pack4(float r0, float r1, float r2, float r3) {
     const __half2 lo = __floats2half2_rn(r0, r1), hi = __floats2half2_rn(r2, r3);
@@ -76,7 +79,7 @@ struct SplOperand {
         return (size_t(g) * blocks + rb) * (size_t(rn) * 64) + size_t(r >> 3) * 512 + (r & 7) * 64 + (((kk >> 3) ^ (r & 7)) << 3) + (kk & 7);
     }
     // The group's sum as the B operand of the GEMM's second term: (hi, lo, hi, lo) with hi + lo = sum / 64 in two fp16
-    // numbers, at contraction index 4 (g % 16) of row `row` of tile (g / 16, row block), the tiles laid out as `at` lays out
+    // numbers. Blocks of 128 rows: at contraction index 4 (g % 16) of row `row` of tile (g / 16, row block), the tiles laid out as `at` lays out
     // the values. (`sums` is that array; the name is kept from the fp32 sums it replaces.)
     __device__ __forceinline__ void put_sum(int row, int g, float sum) const {
         const float mean = sum * 0.015625f;
